@@ -2,30 +2,43 @@
 //
 // Replaces the per-tile potrf task (LAPACKE_dpotrf2 'L',
 // core/src/cpu/adapter_cblas_fp64.cpp:14-22; cusolverDnXpotrf,
-// core/src/gpu/adapter_cublas.cu:9-79).  One CTA of 8 warps factors a
-// bs x bs (bs <= 128) diagonal block; a block smaller than 128 is padded with
-// the identity, so every loop below has a fixed trip count.  Right-looking in
-// 32-wide sub-blocks s = 0..3:
-//   1. warp 0 factors the 32 x 32 diagonal sub-block in registers (lane i
-//      holds row i; the pivot travels by shuffle, the new column of L through
-//      shared memory; branch-free) and forms its inverse X_s column by column
-//      (lane c solves L x = e_c in axpy order, so the 31 updates of a step are
-//      independent);
-//   2. panel solve P = A_rs X_s^T and trailing update A_rr -= P P^T on the
-//      FP64 tensor cores (mma.sync m16n8k8 f64; upper-triangular zero blocks
-//      of X_s are skipped);
-// and the full inverse is assembled block row by block row on the tensor
-// cores,  Linv_s,<s = -X_s (L_s,<s Linv_<s,<s),  Linv_ss = X_s,
-// which turns every later triangular solve against this block (panel trsm,
-// trsv, variance solve) into a GEMM.  Row block s is assembled by warps 1-7
-// while warp 0 runs the pivot chain of sub-block s+1 (the two touch disjoint
-// rows, and no later step reads rows above the current sub-block), so only
-// the last row block's assembly follows the factorisation; each row block of
-// L is written back before its assembly replaces it.  L is written back to the lower
-// triangle only (the strict upper triangle in global memory is never
-// touched, matching dpotrf2('L')).  A non-positive or NaN pivot is recorded
-// in the status word (first failing global row, 1-based); the reference
-// silently returns NaNs instead.
+// core/src/gpu/adapter_cublas.cu:9-79).  One CTA of 16 warps factors a
+// bs x bs (bs <= 128) diagonal block and inverts the factor, which turns every
+// later triangular solve against this block (panel trsm, trsv, variance solve)
+// into a GEMM; a block smaller than 128 is padded with the identity, so every
+// loop below has a fixed trip count.
+//
+// The launch sits on the serial chain of every factorisation (n / 128 of them,
+// one after another), and what bounds it is its own chain: 128 pivots, each
+// the reciprocal of the pivot before it, a product and a shuffle.  So the
+// chain runs alone on warp 0 and everything else beside it, in 32-wide
+// sub-blocks s = 0..3:
+//   warp 0      eliminates the 32 x 32 diagonal sub-block in registers (lane i
+//               holds row i) without square roots, A = L~ D L~^T: the chain
+//               needs one reciprocal per pivot instead of a reciprocal square
+//               root and a scaling, and a pivot column is in shared memory
+//               before its reciprocal is known;
+//   warp 4      follows the pivots a group behind and forms X_s = L_ss^-1 =
+//               D^-1/2 L~^-1 (lane c solves L~ x = e_c; the column of L~ D it
+//               needs is the one warp 0 broadcast), done right after the last
+//               pivot;
+//   all warps   then only what the next chain waits for: the panel rows of
+//               sub-block s+1, P = A X_s^T, and its diagonal A -= P P^T;
+//   the others  beside the next chain, the rest of step s: the panel rows
+//               below, the trailing update, the write-out of L's rows, and
+//               row block s of the inverse,
+//               Linv_s,<s = -X_s T_s, T_s = L_s,<s Linv_<s,  Linv_ss = X_s,
+//               stored to memory from the accumulators, then T_s+1.
+// After the last chain only Linv_3,<3 = -X_3 T_3 is left.  All products run on
+// the FP64 tensor cores (mma.sync m16n8k8 f64).
+// Measured per launch inside the pipelines: 21.3 us FP64, 25.1 us FP32 (43.1
+// and 44.5 with square roots in the chain, the inverse of each sub-block after
+// it and one barrier per phase): loads 1.3 us, a chain window 3 to 4.5 us each,
+// 0.9 us between two of them, 1.3 us after the last.
+// L is written back to the lower triangle only (the strict upper triangle in
+// global memory is never touched, matching dpotrf2('L')).  A non-positive or
+// NaN pivot is recorded in the status word (first failing global row,
+// 1-based); the reference silently returns NaNs instead.
 #include "common.cuh"
 
 namespace gprat_cu
@@ -38,26 +51,25 @@ constexpr int PS = PB + 4;                // smem row stride of the block (confl
 constexpr int SB = 32;                    // sub-block width
 constexpr int XS = SB + 4;                // smem row stride of a sub-block inverse
 constexpr int TS = 3 * SB + 4;            // smem row stride of the assembly temporary
-constexpr int PTHREADS = 256;
+constexpr int HB = SB / 2;                // pivots eliminated in registers at a time
+constexpr int US = SB + 4;                // smem stride of a pivot column (conflict-free fragment loads)
+constexpr int PTHREADS = 512;
 constexpr int NWARPS = PTHREADS / 32;
-constexpr size_t SMEM_DOUBLES = PB * PS + 4 * SB * XS + PB + SB * TS + 2 * SB;
-
-template <typename T>
-struct PairOf;
-template <>
-struct PairOf<double>
-{
-    using type = double2;
-};
-template <>
-struct PairOf<float>
-{
-    using type = float2;
-};
+// A warp's scheduler, with its FP64 pipe, is warp % 4: scheduler 0 runs the
+// chain (warp 0), the inverse that follows it (warp 4) and the data movers
+// (warps 8, 12), the other three the products: a product holds the pipe for 64
+// cycles, a link of the chain for 2, so neither serial part shares a scheduler
+// with them.
+constexpr int CHASE_WARP = 4;
+constexpr int MMA_WARPS = 12;
+constexpr int MOVE_WARPS = 2;
+constexpr int SIDE_WARPS = MMA_WARPS + MOVE_WARPS;
+constexpr size_t SMEM_DOUBLES = PB * PS + 4 * SB * XS + SB * TS + 2 * SB * US + 3 * PB;
+static_assert(SMEM_DOUBLES * sizeof(double) <= 227 * 1024, "shared memory of the diagonal-block kernel");
 
 __device__ __forceinline__ void dmma(double (&c)[4], const double (&a)[4], const double (&b)[2])
 {
-    asm volatile(
+    asm(
         "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
         : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
         : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
@@ -85,114 +97,290 @@ __device__ __forceinline__ void frag_b(double (&b)[2], const double *M, int ld, 
     b[1] = M[(k0 + t + 4) * ld + n0 + g];
 }
 
-// Warp 0: factor the 32 x 32 sub-block at (c0, c0), write L back to smem,
-// and store the pivot reciprocals 1/L_jj in dinv[0..31].
-//
-// Lane i keeps row i in registers; fully unrolled, so every register index is
-// a compile-time constant and pivot j updates exactly the columns j+1..31.
-// Branch-free: a lane's entries above the diagonal receive values that are
-// never read, which keeps the warp converged (per-lane conditional updates
-// compile to divergent branches that cost more than the arithmetic).
-// colbuf (2 x 32 doubles, alternating by pivot, so one __syncwarp per pivot
-// suffices) broadcasts the new column of L; the update reads it in pairs.
-// The next pivot's lane computes its updated diagonal a_j+1,j+1 - l^2 from its
-// own l before the broadcast, and the next pivot's shuffle and rsqrt are
-// issued before the column update, so their latency overlaps it.
-__device__ __forceinline__ void diag_factor_invert(double *a, int c0, int bs, int row0, int *bad, double *dinv,
-                                                   double *colbuf)
+// Stores a 16 x 8 accumulator tile at (m0, n0) of a row-major shared matrix.
+__device__ __forceinline__ void store_tile(double *M, int ld, int m0, int n0, const double (&c)[4], int g, int t)
+{
+    *reinterpret_cast<double2 *>(M + (m0 + g) * ld + n0 + 2 * t) = make_double2(c[0], c[1]);
+    *reinterpret_cast<double2 *>(M + (m0 + g + 8) * ld + n0 + 2 * t) = make_double2(c[2], c[3]);
+}
+
+// Barrier over the nthreads threads that name it (id 0 is __syncthreads), and
+// its arrival without waiting (the producer's half).
+__device__ __forceinline__ void bar_sync(int id, int nthreads)
+{
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(int id, int nthreads)
+{
+    asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
+}
+constexpr int SIDE_BAR = 1;   // the warps beside the chain
+constexpr int HALF_BAR = 2;   // a product warp -> warp 0: the sub-block's last 16 x 16 tile
+constexpr int GROUP_BAR = 3;  // warp 0 -> warp 4, one barrier per pivot group
+
+// The pivots warp 4 waits for at once: groups end after these many.  Short
+// groups at the end, so that warp 4 finishes one pivot behind warp 0.
+constexpr int GROUPS = 6;
+__device__ __forceinline__ constexpr int group_end(int q)
+{
+    constexpr int ends[GROUPS] = { 8, 16, 24, 28, 30, 31 };
+    return ends[q];
+}
+
+// Seeds of the reciprocal and of the reciprocal square root: the hardware's
+// approximations, good to 20 bits or more where neither the argument nor the
+// result is subnormal.
+__device__ __forceinline__ double rcp_seed(double d)
+{
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+    return y;
+}
+__device__ __forceinline__ double rsqrt_seed(double d)
+{
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+    return y;
+}
+
+// 1 / sqrt(d): in the seeds' range the seed y with e = 1 - d y^2 and the
+// third-order step y (1 + e / 2 + 3 e^2 / 8).
+__device__ __forceinline__ double inv_sqrt(double d)
+{
+    if (d > 1e-290 && d < 1e290)
+    {
+        const double y = rsqrt_seed(d);
+        const double e = fma(-(d * y), y, 1.0);
+        return fma(y * e, fma(e, 0.375, 0.5), y);
+    }
+    return rsqrt(d);
+}
+
+// The range the seeds (and the squares of a pivot column) are used in, by the
+// sub-block's current diagonal, which bounds its pivots and columns.  A pivot
+// that falls below MIN_PIVOT from there lost 170 decimal places to
+// cancellation and is reported like a non-positive one.
+__device__ __forceinline__ bool seeds_apply(double diag) { return diag > 1e-120 && diag < 1e150; }
+constexpr double MIN_PIVOT = 1e-290;
+
+// Warp 0: A = L~ D L~^T of the 32 x 32 sub-block at (c0, c0), lane i holding row
+// i, 16 columns at a time; the last 16 x 16 tile is updated with the first 16
+// pivots on the tensor cores (in registers it would double the chain's
+// instructions, which is what the shared loads of a 32-column step cost:
+// measured 143 against 95 cycles per pivot).  Leaves for warp 4 and the
+// write-out: u[j][i] = (L~ D)_ij (column j as it stood when it became the
+// pivot column), the pivots d and their reciprocals.  Fully unrolled, so every
+// register index is a compile-time constant, and branch-free: a lane's entries
+// above the diagonal receive values that are never read, which keeps the warp
+// converged.
+// The chain from pivot to pivot, d' = a - u^2 / d on lane j+1 and a shuffle:
+// with the seed y and e = 1 - d y, 1 / d = y + y (e + e^2) (third order, the
+// error e^3 is below the last place), so d' = (a - u^2 y) - (u^2 y)(e + e^2),
+// whose operands but the last are ready one step earlier.  FAST false (entries
+// out of the seeds' range): divisions.
+template <bool FAST>
+__device__ __forceinline__ void pivot_chain(double *a, int c0, bool wait_tile, double *u, double *piv, double *pinv)
 {
     const int lane = threadIdx.x & 31;
-    double r[SB];  // r[c] = A[lane][c0 + c]
-    {
-        const double *arow = a + (c0 + lane) * PS + c0;
+    const int g = lane >> 2, t = lane & 3;
 #pragma unroll
-        for (int c = 0; c < SB; ++c)
-        {
-            r[c] = (c <= lane) ? arow[c] : 0.0;
-        }
-    }
-    int first_bad = 0;
-    double ajj = __shfl_sync(0xffffffffu, r[0], 0);  // the current pivot's updated diagonal entry
-    double inv = rsqrt(ajj);
-#pragma unroll
-    for (int j = 0; j < SB; ++j)
+    for (int h = 0; h < 2; ++h)
     {
-        double *cb = colbuf + (j & 1) * SB;
-        first_bad = (first_bad == 0 && !(ajj > 0.0) && c0 + j < bs) ? row0 + c0 + j + 1 : first_bad;
-        const double l = (lane == j) ? ajj * inv : r[j] * inv;  // L[lane][j] for lane >= j
-        cb[lane] = l;
-        a[(c0 + lane) * PS + c0 + j] = l;  // above the diagonal: a value nobody reads
-        if (lane == 0)
+        if (h == 1)
         {
-            dinv[j] = inv;
-        }
-        if (j + 1 < SB)
-        {
-            const double dnext = r[j + 1] - l * l;  // lane j+1: the next pivot
+            // the last 16 x 16 tile: A22 -= (U21 D^-1) U21^T
+            if (wait_tile)
+            {
+                bar_sync(HALF_BAR, 64);
+            }
+            double *c = a + (c0 + HB + g) * PS + c0 + HB + 2 * t;
+            double af[2][4], bf[2][2][2], cf[2][4];
+#pragma unroll
+            for (int kk = 0; kk < 2; ++kk)
+            {
+                const double *k0 = u + (8 * kk + t) * US + HB, *k1 = k0 + 4 * US;
+                const double p0 = pinv[8 * kk + t], p1 = pinv[8 * kk + t + 4];
+                af[kk][0] = -k0[g] * p0;
+                af[kk][1] = -k0[g + 8] * p0;
+                af[kk][2] = -k1[g] * p1;
+                af[kk][3] = -k1[g + 8] * p1;
+#pragma unroll
+                for (int n = 0; n < 2; ++n)
+                {
+                    bf[kk][n][0] = k0[8 * n + g];
+                    bf[kk][n][1] = k1[8 * n + g];
+                }
+            }
+#pragma unroll
+            for (int n = 0; n < 2; ++n)
+            {
+                cf[n][0] = c[8 * n];
+                cf[n][1] = c[8 * n + 1];
+                cf[n][2] = c[8 * PS + 8 * n];
+                cf[n][3] = c[8 * PS + 8 * n + 1];
+            }
+#pragma unroll
+            for (int kk = 0; kk < 2; ++kk)
+            {
+#pragma unroll
+                for (int n = 0; n < 2; ++n)
+                {
+                    dmma(cf[n], af[kk], bf[kk][n]);
+                }
+            }
+            store_tile(a, PS, c0 + HB, c0 + HB, cf[0], g, t);
+            store_tile(a, PS, c0 + HB, c0 + HB + 8, cf[1], g, t);
             __syncwarp();
-            // the next pivot's shuffle and rsqrt are independent of the column
-            // update below and overlap it
-            ajj = __shfl_sync(0xffffffffu, dnext, j + 1);
-            inv = rsqrt(ajj);
-            int c = j + 1;
-            if (c & 1)
+        }
+        double r[HB];  // r[c] = A[lane][c0 + 16 h + c]
+        const double *arow = a + (c0 + lane) * PS + c0 + h * HB;
+#pragma unroll
+        for (int c = 0; c < HB; ++c)
+        {
+            r[c] = (h * HB + c <= lane) ? arow[c] : 0.0;
+        }
+        double d = __shfl_sync(0xffffffffu, r[0], h * HB);  // the current pivot
+#pragma unroll
+        for (int jj = 0; jj < HB; ++jj)
+        {
+            const int j = h * HB + jj;
+            double *cb = u + j * US;
+            cb[lane] = r[jj];
+            const double y = FAST ? rcp_seed(d) : 1.0 / d;
+            double dinv = y, dnext = 0.0;
+            if (FAST)
             {
-                r[c] -= l * cb[c];
-                ++c;
+                const double e = fma(-d, y, 1.0);
+                const double ee = fma(e, e, e);
+                dinv = fma(y, ee, y);
+                if (jj + 1 < HB)
+                {
+                    const double q = r[jj] * r[jj] * y;
+                    dnext = fma(-q, ee, r[jj + 1] - q);
+                }
+            }
+            else if (jj + 1 < HB)
+            {
+                dnext = fma(-r[jj] * y, r[jj], r[jj + 1]);
+            }
+            if (lane == 0)
+            {
+                piv[j] = d;
+                pinv[j] = dinv;
             }
 #pragma unroll
-            for (; c < SB; c += 2)
+            for (int q = 0; q < GROUPS; ++q)
             {
-                const double2 v = *reinterpret_cast<const double2 *>(cb + c);
-                r[c] -= l * v.x;
-                r[c + 1] -= l * v.y;
+                if (group_end(q) == j + 1)
+                {
+                    bar_arrive(GROUP_BAR + q, 64);
+                }
+            }
+            if (jj + 1 < HB)
+            {
+                d = __shfl_sync(0xffffffffu, dnext, j + 1);
+                const double w = r[jj] * dinv;  // L~[lane][j]
+                __syncwarp();
+                int c = jj + 1;
+                if (c & 1)
+                {
+                    r[c] = fma(-w, cb[h * HB + c], r[c]);
+                    ++c;
+                }
+#pragma unroll
+                for (; c < HB; c += 2)
+                {
+                    const double2 v = *reinterpret_cast<const double2 *>(cb + h * HB + c);
+                    r[c] = fma(-w, v.x, r[c]);
+                    r[c + 1] = fma(-w, v.y, r[c + 1]);
+                }
             }
         }
-    }
-    if (lane == 0 && first_bad != 0 && *bad == 0)
-    {
-        *bad = first_bad;
+        __syncwarp();
     }
 }
 
-// All 8 warps: X = L^-1 of the factored 32 x 32 sub-block at (c0, c0), zero
-// above the diagonal, into xinv.  Warp w solves columns 4w .. 4w+3; lane i owns
-// row i and the four columns' x_i.  The system is scaled to a unit diagonal
-// first (row i of L and of the right-hand side times 1/L_ii), so step k is one
-// shuffle of the final x_k and one FMA on the lanes below (their strictly
-// lower entries; every other coefficient is zero).  Fully unrolled (32 short
-// steps) and branch-free.
-__device__ __forceinline__ void diag_inverse_all_warps(const double *a, int c0, const double *dinv, double *xinv)
+// Warp 4: X~ = L~^-1 (zero above the diagonal) of the sub-block warp 0 is
+// eliminating, lane c column c, 16 rows at a time (the first half's part in the
+// second half's rows on the tensor cores).  L^-1 = D^-1/2 X~: its readers scale
+// the rows.  Waits for a group of pivots at a time.
+__device__ __forceinline__ void chase_inverse(const double *u, const double *pinv, double *xinv)
 {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    double lrow[SB];
-    const double *arow = a + (c0 + lane) * PS + c0;
-    const double di = dinv[lane];
+    const int lane = threadIdx.x & 31;
+    const int g = lane >> 2, t = lane & 3;
 #pragma unroll
-    for (int c = 0; c < SB; ++c)
+    for (int h = 0; h < 2; ++h)
     {
-        lrow[c] = (c < lane) ? arow[c] * di : 0.0;
-    }
-    double x[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-    {
-        x[q] = (lane == 4 * warp + q) ? di : 0.0;
-    }
-#pragma unroll
-    for (int k = 0; k < SB; ++k)
-    {
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
+        double x[HB];
+        if (h == 0)
         {
-            const double xk = __shfl_sync(0xffffffffu, x[q], k);
-            x[q] -= lrow[k] * xk;
-        }
-    }
 #pragma unroll
-    for (int q = 0; q < 4; ++q)
-    {
-        xinv[lane * XS + 4 * warp + q] = x[q];
+            for (int i = 0; i < HB; ++i)
+            {
+                x[i] = (i == lane) ? 1.0 : 0.0;
+            }
+        }
+        else
+        {
+            // rows 16 .. 31 of columns 0 .. 15: the first half's share,
+            // -L~21 X~11 (L~_ij = u_ij / d_j), through their place in xinv
+            __syncwarp();
+            double cf[2][4] = {};
+#pragma unroll
+            for (int kk = 0; kk < 2; ++kk)
+            {
+                const double *k0 = u + (8 * kk + t) * US + HB, *k1 = k0 + 4 * US;
+                const double p0 = -pinv[8 * kk + t], p1 = -pinv[8 * kk + t + 4];
+                const double af[4] = { k0[g] * p0, k0[g + 8] * p0, k1[g] * p1, k1[g + 8] * p1 };
+#pragma unroll
+                for (int n = 0; n < 2; ++n)
+                {
+                    double bf[2];
+                    frag_b(bf, xinv, XS, 8 * n, 8 * kk, g, t);
+                    dmma(cf[n], af, bf);
+                }
+            }
+            store_tile(xinv, XS, HB, 0, cf[0], g, t);
+            store_tile(xinv, XS, HB, 8, cf[1], g, t);
+            __syncwarp();
+#pragma unroll
+            for (int i = 0; i < HB; ++i)
+            {
+                x[i] = (lane < HB) ? xinv[(HB + i) * XS + lane] : (HB + i == lane ? 1.0 : 0.0);
+            }
+        }
+#pragma unroll
+        for (int jj = 0; jj < HB; ++jj)
+        {
+            const int j = h * HB + jj;
+#pragma unroll
+            for (int q = 0; q < GROUPS; ++q)
+            {
+                if ((q == 0 ? 0 : group_end(q - 1)) == j)  // (the last pivot's own column is not needed)
+                {
+                    bar_sync(GROUP_BAR + q, 64);
+                }
+            }
+            const double *cb = u + j * US + h * HB;
+            xinv[j * XS + lane] = x[jj];
+            if (jj + 1 < HB)
+            {
+                const double w = x[jj] * pinv[j];
+                int c = jj + 1;
+                if (c & 1)
+                {
+                    x[c] = fma(-w, cb[c], x[c]);
+                    ++c;
+                }
+#pragma unroll
+                for (; c < HB; c += 2)
+                {
+                    const double2 v = *reinterpret_cast<const double2 *>(cb + c);
+                    x[c] = fma(-w, v.x, x[c]);
+                    x[c + 1] = fma(-w, v.y, x[c + 1]);
+                }
+            }
+        }
     }
 }
 
@@ -202,181 +390,6 @@ __device__ __forceinline__ void cp_async16_zfill(void *smem, const void *gmem, i
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(gmem), "r"(bytes) : "memory");
 }
 
-// Offset (in 16-byte chunks) of row i in the packed FP32 staging of a lower
-// triangle whose row r holds r / 4 + 1 chunks (columns 0 .. 4 (r / 4) + 3).
-__device__ __forceinline__ int staged_row_chunks(int i)
-{
-    const int q = i >> 2, r = i & 3;
-    return (q + 1) * (2 * q + r);
-}
-
-// Loads the lower triangle of the block (rows < bs) with 16-byte cp.async
-// copies, then pads: the strict upper triangle is zero and rows >= bs are
-// identity rows.  Needs A and lda * sizeof(T) 16-byte aligned.  Every copy
-// stops at column i of its row (the rest of the chunk is zero-filled), so
-// nothing right of the block's diagonal is read.
-//   FP64: rows go straight to their place in sa;
-//   FP32: rows are packed into `stage` (2112 chunks, 33 KB), then widened.
-template <typename T>
-__device__ __forceinline__ void load_lower_async(const T *__restrict__ A, int64_t lda, int bs, double *sa,
-                                                 double *stage)
-{
-    constexpr int CH = 16 / sizeof(T);  // elements per chunk
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float *st32 = reinterpret_cast<float *>(stage);
-    for (int i = warp; i < bs; i += NWARPS)
-    {
-        const int nchunks = i / CH + 1;
-        for (int k = lane; k < nchunks; k += 32)
-        {
-            const int c = k * CH;
-            const int bytes = min(CH, i + 1 - c) * static_cast<int>(sizeof(T));
-            void *dst = (sizeof(T) == 8) ? static_cast<void *>(sa + i * PS + c)
-                                         : static_cast<void *>(st32 + 4 * (staged_row_chunks(i) + k));
-            cp_async16_zfill(dst, A + static_cast<int64_t>(i) * lda + c, bytes);
-        }
-    }
-    asm volatile("cp.async.wait_all;\n" ::: "memory");
-    __syncthreads();
-    for (int q = threadIdx.x; q < PB * PB / 2; q += PTHREADS)
-    {
-        const int i = q >> 6, c = 2 * (q & 63);
-        double v0 = (i == c) ? 1.0 : 0.0, v1 = (i == c + 1) ? 1.0 : 0.0;
-        if (i < bs && c <= i)
-        {
-            if (sizeof(T) == 8)
-            {
-                const double2 w = *reinterpret_cast<const double2 *>(sa + i * PS + c);
-                v0 = w.x;
-                v1 = (c + 1 <= i) ? w.y : 0.0;
-            }
-            else
-            {
-                const float *row = st32 + 4 * staged_row_chunks(i);
-                v0 = static_cast<double>(row[c]);
-                v1 = (c + 1 <= i) ? static_cast<double>(row[c + 1]) : 0.0;
-            }
-        }
-        *reinterpret_cast<double2 *>(sa + i * PS + c) = make_double2(v0, v1);
-    }
-}
-
-// Barrier over the nthreads threads of warps first .. (a named barrier; id 0
-// with every thread is __syncthreads).
-__device__ __forceinline__ void bar_sync(int id, int nthreads)
-{
-    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
-}
-
-// Inverse of row block s (rows 32s .. 32s + 31), in place in sa, whose rows
-// < 32s already hold Linv:  Linv_s,<s = -X_s (L_s,<s Linv_<s,<s),  Linv_ss = X_s.
-// Run by nwarps warps starting at first_warp; barrier bar_id (over those
-// warps) separates the reads of L_s,<s from the writes that replace it.
-__device__ __forceinline__ void assemble_row_block(double *sa, const double *xs, double *tbuf, int s, int first_warp,
-                                                   int nwarps, int bar_id)
-{
-    const int lane = threadIdx.x & 31, w = (threadIdx.x >> 5) - first_warp;
-    const int g = lane >> 2, t = lane & 3;
-    const int c0 = s * SB;
-    if (s > 0)
-    {
-        // T = L[c0.., 0..c0) Linv[0..c0, 0..c0)   (32 x c0; Linv lower: k >= n)
-        const int nt_count = c0 / 8;
-        for (int tile = w; tile < 2 * nt_count; tile += nwarps)
-        {
-            const int mi = tile / nt_count, nt = tile % nt_count;
-            double cf[4] = { 0.0, 0.0, 0.0, 0.0 };
-            for (int kk = nt; kk < nt_count; ++kk)
-            {
-                double af[4], bf[2];
-                frag_a(af, sa, PS, c0 + 16 * mi, 8 * kk, g, t);
-                frag_b(bf, sa, PS, 8 * nt, 8 * kk, g, t);
-                dmma(cf, af, bf);
-            }
-            double *c = tbuf + (16 * mi + g) * TS + 8 * nt + 2 * t;
-            c[0] = cf[0];
-            c[1] = cf[1];
-            c[8 * TS] = cf[2];
-            c[8 * TS + 1] = cf[3];
-        }
-        bar_sync(bar_id, nwarps * 32);
-        // Linv[c0.., 0..c0) = -X T   (X lower: k <= row)
-        for (int tile = w; tile < 2 * nt_count; tile += nwarps)
-        {
-            const int mi = tile / nt_count, nt = tile % nt_count;
-            double cf[4] = { 0.0, 0.0, 0.0, 0.0 };
-#pragma unroll
-            for (int kk = 0; kk < 4; ++kk)
-            {
-                if (kk <= 2 * mi + 1)
-                {
-                    double af[4], bf[2];
-                    frag_a(af, xs, XS, 16 * mi, 8 * kk, g, t);
-                    frag_b(bf, tbuf, TS, 8 * nt, 8 * kk, g, t);
-#pragma unroll
-                    for (int e = 0; e < 4; ++e)
-                    {
-                        af[e] = -af[e];
-                    }
-                    dmma(cf, af, bf);
-                }
-            }
-            double *c = sa + (c0 + 16 * mi + g) * PS + 8 * nt + 2 * t;
-            c[0] = cf[0];
-            c[1] = cf[1];
-            c[8 * PS] = cf[2];
-            c[8 * PS + 1] = cf[3];
-        }
-    }
-    // diagonal block: X_s (zero above the diagonal)
-    for (int q = w * 32 + lane; q < SB * SB; q += nwarps * 32)
-    {
-        const int i = q / SB, j = q % SB;
-        sa[(c0 + i) * PS + c0 + j] = (j <= i) ? xs[i * XS + j] : 0.0;
-    }
-}
-
-// Writes row block c0 .. c0 + 31 of L (lower triangle with the diagonal, rows
-// < bs) back to A: in pairs of columns when the block is 16-byte aligned,
-// else element by element.
-template <typename T>
-__device__ __forceinline__ void write_l_block(T *A, int64_t lda, const double *sa, int c0, int bs, bool aligned)
-{
-    using Pair = typename PairOf<T>::type;
-    for (int q = threadIdx.x; q < SB * (PB / 2); q += PTHREADS)
-    {
-        const int i = c0 + (q >> 6), c = 2 * (q & 63);
-        if (i >= bs || c > i)
-        {
-            continue;
-        }
-        T *dst = A + static_cast<int64_t>(i) * lda + c;
-        if (aligned)
-        {
-            const double2 v = *reinterpret_cast<const double2 *>(sa + i * PS + c);
-            if (c + 1 <= i)
-            {
-                Pair w;
-                w.x = static_cast<T>(v.x);
-                w.y = static_cast<T>(v.y);
-                *reinterpret_cast<Pair *>(dst) = w;
-            }
-            else
-            {
-                dst[0] = static_cast<T>(v.x);
-            }
-        }
-        else
-        {
-            dst[0] = static_cast<T>(sa[i * PS + c]);
-            if (c + 1 <= i)
-            {
-                dst[1] = static_cast<T>(sa[i * PS + c + 1]);
-            }
-        }
-    }
-}
-
 // True when the block and its rows start on 16-byte boundaries.
 template <typename T>
 __device__ __forceinline__ bool aligned16(const T *A, int64_t lda)
@@ -384,202 +397,526 @@ __device__ __forceinline__ bool aligned16(const T *A, int64_t lda)
     return ((reinterpret_cast<uintptr_t>(A) | static_cast<uintptr_t>(lda * sizeof(T))) & 15) == 0;
 }
 
+// Rows [R_LO, R_HI) of the block's lower triangle into shared memory, all
+// threads.  Nothing right of the block's diagonal is read; shared words right
+// of it may receive zeros and are never read as part of L.  FP64 blocks on
+// 16-byte boundaries: cp.async (the caller waits); everything else (FP32 is
+// widened): plain loads, those of eight rows issued before the first is used.
+template <int R_LO, int R_HI, typename T>
+__device__ __forceinline__ void load_rows(const T *A, int64_t lda, bool al, int bs, double *sa)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int ROWS = (R_HI - R_LO) / NWARPS;  // per warp
+    if (sizeof(T) == 8 && al)
+    {
+#pragma unroll
+        for (int k = 0; k < ROWS; ++k)
+        {
+            const int i = R_LO + NWARPS * k + warp;
+#pragma unroll
+            for (int c0 = 0; c0 < R_LO + NWARPS * (k + 1); c0 += 64)
+            {
+                const int c = c0 + 2 * lane;
+                if (c <= i && i < bs)
+                {
+                    cp_async16_zfill(sa + i * PS + c, A + static_cast<int64_t>(i) * lda + c, min(2, i + 1 - c) * 8);
+                }
+            }
+        }
+    }
+    else
+    {
+#pragma unroll
+        for (int k0 = 0; k0 < ROWS; k0 += 8)
+        {
+            T v[8][4];
+#pragma unroll
+            for (int q = 0; q < 8 && k0 + q < ROWS; ++q)
+            {
+                const int i = R_LO + NWARPS * (k0 + q) + warp;
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                {
+                    const int c = lane + 32 * k;
+                    v[q][k] = (c <= i && i < bs) ? A[static_cast<int64_t>(i) * lda + c] : T(0);
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < 8 && k0 + q < ROWS; ++q)
+            {
+                const int i = R_LO + NWARPS * (k0 + q) + warp;
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                {
+                    sa[i * PS + lane + 32 * k] = static_cast<double>(v[q][k]);
+                }
+            }
+        }
+    }
+    // identity rows below a block smaller than 128
+    for (int i = max(R_LO, bs); i < R_HI; ++i)
+    {
+        if ((i & (NWARPS - 1)) == warp)
+        {
+            for (int c = lane; c <= i; c += 32)
+            {
+                sa[i * PS + c] = (i == c) ? 1.0 : 0.0;
+            }
+        }
+    }
+}
+
+// One element pair (i, c), (i, c + 1) of an output matrix, c even: columns
+// <= c_last are stored, as a pair where `pair` allows it.
+template <typename T>
+struct PairOf;
+template <>
+struct PairOf<double>
+{
+    using type = double2;
+};
+template <>
+struct PairOf<float>
+{
+    using type = float2;
+};
+template <typename T>
+__device__ __forceinline__ void store_pair(T *M, int64_t ld, int i, int c, int c_last, bool pair, double v0, double v1)
+{
+    using Pair = typename PairOf<T>::type;
+    T *dst = M + static_cast<int64_t>(i) * ld + c;
+    if (pair && c + 1 <= c_last)
+    {
+        Pair w;
+        w.x = static_cast<T>(v0);
+        w.y = static_cast<T>(v1);
+        *reinterpret_cast<Pair *>(dst) = w;
+        return;
+    }
+    if (c <= c_last)
+    {
+        dst[0] = static_cast<T>(v0);
+    }
+    if (c + 1 <= c_last)
+    {
+        dst[1] = static_cast<T>(v1);
+    }
+}
+
+// Where the inverse goes: FP64 and / or FP32 (either may be null), rows and
+// columns < bs.
+struct InverseOut
+{
+    double *f64;
+    int64_t ld64;
+    float *f32;
+    int64_t ld32;
+    int bs;
+    __device__ __forceinline__ void pair(int i, int c, double v0, double v1) const
+    {
+        if (i >= bs || c >= bs)
+        {
+            return;
+        }
+        if (f64 != nullptr)
+        {
+            store_pair(f64, ld64, i, c, bs - 1, true, v0, v1);
+        }
+        if (f32 != nullptr)
+        {
+            store_pair(f32, ld32, i, c, bs - 1, true, v0, v1);
+        }
+    }
+};
+
+// Row block s of the inverse left of its diagonal block: -X_s T_s (X_s = D^-1/2 X~_s), 16 x 16
+// tiles over nwarps warps (this one is number w), to memory and, when
+// keep, into sa in place of L_s,<s.
+__device__ __forceinline__ void inverse_row_block(const InverseOut &out, double *sa, bool keep, const double *xs, const double *rsq,
+                                                  const double *tbuf, int s, int w, int nwarps, int g, int t)
+{
+    const int c0 = s * SB;
+    for (int tile = w; tile < 4 * s; tile += nwarps)
+    {
+        const int mi = tile / (2 * s), n0 = 16 * (tile % (2 * s));
+        double cf[2][4] = {};
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk)
+        {
+            if (kk <= 2 * mi + 1)  // X is lower triangular
+            {
+                double af[4];
+                frag_a(af, xs, XS, 16 * mi, 8 * kk, g, t);
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                {
+                    double bf[2];
+                    frag_b(bf, tbuf, TS, n0 + 8 * h, 8 * kk, g, t);
+                    dmma(cf[h], af, bf);
+                }
+            }
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+        {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+            {
+                cf[h][e] *= -rsq[c0 + 16 * mi + g + (e >> 1) * 8];
+            }
+            const int i = c0 + 16 * mi + g, c = n0 + 8 * h + 2 * t;
+            out.pair(i, c, cf[h][0], cf[h][1]);
+            out.pair(i + 8, c, cf[h][2], cf[h][3]);
+            if (keep)
+            {
+                store_tile(sa, PS, c0 + 16 * mi, n0 + 8 * h, cf[h], g, t);
+            }
+        }
+    }
+}
+
+// A -= P P^T on the 16 x 16 tile at (m0, n0), P the 32 columns from p0.
+__device__ __forceinline__ void trailing_tile(double *sa, int m0, int n0, int p0, int g, int t)
+{
+    double cf[2][4] = {};
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk)
+    {
+        double af[4];
+        frag_a(af, sa, PS, m0, p0 + 8 * kk, g, t);
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+        {
+            double bf[2];
+            frag_bt(bf, sa, PS, n0 + 8 * h, p0 + 8 * kk, g, t);
+            dmma(cf[h], af, bf);
+        }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+    {
+        const double *c = sa + (m0 + g) * PS + n0 + 8 * h + 2 * t;
+        const double2 v0 = *reinterpret_cast<const double2 *>(c);
+        const double2 v1 = *reinterpret_cast<const double2 *>(c + 8 * PS);
+        const double tile[4] = { v0.x - cf[h][0], v0.y - cf[h][1], v1.x - cf[h][2], v1.y - cf[h][3] };
+        store_tile(sa, PS, m0, n0 + 8 * h, tile, g, t);
+    }
+}
+
+// T_s = L_s,<s Linv_<s  (32 x 32 s; Linv lower triangular: k >= n), 16 x 16
+// tiles, those with the most products first.
+__device__ __forceinline__ void inverse_temporary(double *tbuf, const double *sa, int s, int w, int nwarps, int g,
+                                                  int t)
+{
+    for (int tile = w; tile < 4 * s; tile += nwarps)
+    {
+        const int mi = tile & 1, p = tile >> 1;
+        double cf[2][4] = {};
+#pragma unroll 2
+        for (int kk = 2 * p; kk < 4 * s; ++kk)
+        {
+            double af[4];
+            frag_a(af, sa, PS, s * SB + 16 * mi, 8 * kk, g, t);
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+            {
+                double bf[2];
+                frag_b(bf, sa, PS, 16 * p + 8 * h, 8 * kk, g, t);
+                dmma(cf[h], af, bf);
+            }
+        }
+        store_tile(tbuf, TS, 16 * mi, 16 * p, cf[0], g, t);
+        store_tile(tbuf, TS, 16 * mi, 16 * p + 8, cf[1], g, t);
+    }
+}
+
 // T: element type of the block in global memory (FP64, or FP32 for the
 // mixed path, which then also receives Linv in FP32 and the FP64 diagonal of L).
 template <typename T>
-__global__ void __launch_bounds__(PTHREADS, 1) potrf_inv_kernel(T *__restrict__ A, int64_t lda, int bs, int row0,
-                                                                double *__restrict__ Linv, int64_t ldi,
-                                                                float *__restrict__ Linv32, int64_t ldi32,
+__global__ void __launch_bounds__(PTHREADS, 1) potrf_inv_kernel(T *A, int64_t lda, int bs, int row0, double *Linv,
+                                                                int64_t ldi, float *Linv32, int64_t ldi32,
                                                                 double *__restrict__ diag_out,
                                                                 DeviceStatus *__restrict__ status, int write_l)
 {
-    extern __shared__ double sa[];  // [PB][PS]
-    double *xall = sa + PB * PS;    // 4 x [SB][XS] sub-block inverses
-    double *dinv = xall + 4 * SB * XS;       // [PB] pivot reciprocals
-    double *tbuf = dinv + PB;                // [SB][TS]
-    double *colbuf = tbuf + SB * TS;         // [2][SB] column broadcast of the diagonal factorisation
+    extern __shared__ __align__(16) double sa[];  // [PB][PS]
+    double *xall = sa + PB * PS;         // 4 x [SB][XS] sub-block inverses
+    double *tbuf = xall + 4 * SB * XS;   // [SB][TS]
+    double *ubuf = tbuf + SB * TS;       // 2 x [SB][US] pivot columns, alternating by sub-block
+    double *piv = ubuf + 2 * SB * US;    // [PB] pivots
+    double *pinv = piv + PB;             // [PB] their reciprocals
+    double *rsq = pinv + PB;             // [PB] their reciprocal square roots (from the step after the pivots' on)
     __shared__ int bad;
+    __shared__ double min_pivot;
     const int tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
+    const bool mover = warp > CHASE_WARP && (warp & 3) == 0;
+    const int mma_w = warp - 1 - (warp >> 2);                         // number among the product warps
+    const int move_w = (warp >> 2) - 2, move_t = 32 * move_w + lane;  // among the data movers
+    const InverseOut out{ Linv, ldi, Linv32, ldi32, bs };
     if (tid == 0)
     {
         bad = 0;
     }
     pdl_wait();  // the previous kernel's results are visible from here on
-    if (aligned16(A, lda))
-    {
-        load_lower_async(A, lda, bs, sa, xall);
-    }
-    else
-    {
-        // unaligned block: element loads of the lower triangle, identity padding
-        for (int q = tid; q < PB * PB; q += PTHREADS)
-        {
-            const int i = q >> 7, c = q & (PB - 1);
-            sa[i * PS + c] = (i < bs && c <= i) ? static_cast<double>(A[static_cast<int64_t>(i) * lda + c])
-                                                : ((i == c) ? 1.0 : 0.0);
-        }
-    }
+    const bool al = aligned16(A, lda);
+    // the first sub-block's rows ahead of the rest: its chain starts on them
+    load_rows<0, SB>(A, lda, al, bs, sa);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    load_rows<SB, PB>(A, lda, al, bs, sa);
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 1;\n" ::: "memory");
     __syncthreads();
 
-    const bool al = aligned16(A, lda);
+    // L's sub-block s (its columns u scaled by 1 / sqrt(d)) and diagonal, to
+    // memory, by this thread as number me of count
+    auto write_diag = [&](int s, int me, int count)
+    {
+        const double *u = ubuf + (s & 1) * SB * US;
+        const int c0 = s * SB;
+        for (int q = me; write_l && q < SB * SB / 2; q += count)
+        {
+            const int i = q >> 4, c = 2 * (q & 15);
+            if (c <= i && c0 + i < bs)
+            {
+                store_pair(A, lda, c0 + i, c0 + c, c0 + i, al, u[c * US + i] * rsq[c0 + c],
+                           u[(c + 1) * US + i] * rsq[c0 + c + 1]);
+            }
+        }
+        for (int j = me; diag_out != nullptr && j < SB; j += count)
+        {
+            if (c0 + j < bs)
+            {
+                diag_out[c0 + j] = piv[c0 + j] * rsq[c0 + j];
+            }
+        }
+    };
+    // one warp: 1 / sqrt of sub-block s's pivots, and the first that is not positive
+    auto finish_pivots = [&](int s)
+    {
+        const double d = piv[s * SB + lane];
+        rsq[s * SB + lane] = inv_sqrt(d);
+        const unsigned wrong = __ballot_sync(0xffffffffu, !(d > min_pivot) && s * SB + lane < bs);
+        if (lane == 0 && wrong != 0 && bad == 0)
+        {
+            bad = row0 + s * SB + __ffs(wrong);
+        }
+    };
+    // the inverse's diagonal block s, to memory and (keep) into sa
+    auto write_xs = [&](int s, bool keep, int me, int count)
+    {
+        const double *xs = xall + s * SB * XS;
+        const int c0 = s * SB;
+        for (int q = me; q < SB * SB / 2; q += count)
+        {
+            const int i = q >> 4, c = 2 * (q & 15);
+            double2 v = *reinterpret_cast<const double2 *>(xs + i * XS + c);
+            v.x *= rsq[c0 + i];
+            v.y *= rsq[c0 + i];
+            out.pair(c0 + i, c0 + c, v.x, v.y);
+            if (keep)
+            {
+                *reinterpret_cast<double2 *>(sa + (c0 + i) * PS + c0 + c) = v;
+            }
+        }
+    };
+
 #pragma unroll 1
     for (int s = 0; s < 4; ++s)
     {
         const int c0 = s * SB;
-        double *xs = xall + s * SB * XS;
+        const double *xs = xall + s * SB * XS;
+        double *u = ubuf + (s & 1) * SB * US;
         if (warp == 0)
         {
-            diag_factor_invert(sa, c0, bs, row0, &bad, dinv + c0, colbuf);
-        }
-        else if (s > 0)
-        {
-            // the previous row block's inverse, beside this sub-block's pivots
-            // (disjoint rows; later steps never read rows above c0)
-            assemble_row_block(sa, xall + (s - 1) * SB * XS, tbuf, s - 1, 1, NWARPS - 1, 1);
-        }
-        __syncthreads();
-        diag_inverse_all_warps(sa, c0, dinv + c0, xs);
-        // row block s of L is final: write it back (and its diagonal) before
-        // the assembly replaces it with Linv
-        if (write_l)
-        {
-            write_l_block(A, lda, sa, c0, bs, al);
-        }
-        if (diag_out != nullptr && tid < SB && c0 + tid < bs)
-        {
-            diag_out[c0 + tid] = sa[(c0 + tid) * PS + c0 + tid];
-        }
-        __syncthreads();
-        if (s == 3)
-        {
-            break;
-        }
-        const int r0 = c0 + SB;
-        const int R = PB - r0;  // 96, 64, 32 rows below
-        // panel: P = A[r0.., c0..c0+31] X^T  (warp w owns rows r0 + 16w .. +15)
-        if (warp < R / 16)
-        {
-            const int m0 = r0 + 16 * warp;
-            double af[4][4];
-#pragma unroll
-            for (int kk = 0; kk < 4; ++kk)
+            if (__all_sync(0xffffffffu, seeds_apply(sa[(c0 + lane) * PS + c0 + lane])))
             {
-                frag_a(af[kk], sa, PS, m0, c0 + 8 * kk, g, t);
+                min_pivot = MIN_PIVOT;
+                pivot_chain<true>(sa, c0, s > 0, u, piv + c0, pinv + c0);
             }
-            double cf[4][4];
-#pragma unroll
-            for (int nt = 0; nt < 4; ++nt)
+            else
             {
-#pragma unroll
-                for (int e = 0; e < 4; ++e)
-                {
-                    cf[nt][e] = 0.0;
-                }
-#pragma unroll
-                for (int kk = 0; kk <= nt; ++kk)  // X^T is zero where k > n
-                {
-                    double bf[2];
-                    frag_bt(bf, xs, XS, 8 * nt, 8 * kk, g, t);
-                    dmma(cf[nt], af[kk], bf);
-                }
-            }
-            __syncwarp();
-#pragma unroll
-            for (int nt = 0; nt < 4; ++nt)
-            {
-                double *c = sa + (m0 + g) * PS + c0 + 8 * nt + 2 * t;
-                c[0] = cf[nt][0];
-                c[1] = cf[nt][1];
-                c[8 * PS] = cf[nt][2];
-                c[8 * PS + 1] = cf[nt][3];
+                min_pivot = 0.0;
+                pivot_chain<false>(sa, c0, s > 0, u, piv + c0, pinv + c0);
             }
         }
-        __syncthreads();
-        // trailing update of the lower tiles: A[r0.., r0..] -= P P^T
+        else if (warp == CHASE_WARP)
         {
-            const int mt = R / 16;
-            const int ntiles = mt * (mt + 1);  // sum over mi of (2 mi + 2)
-            for (int tile = warp; tile < ntiles; tile += NWARPS)
+            chase_inverse(u, pinv + c0, xall + s * SB * XS);
+        }
+        else if (s == 0)
+        {
+            // zeros above the inverse's diagonal blocks
+            for (int i = mover ? MMA_WARPS + move_w : mma_w; i < 3 * SB; i += SIDE_WARPS)
             {
-                // tile -> (mi, ni) with ni <= 2 mi + 1
-                int mi = 0, base = 0;
-                while (base + 2 * mi + 2 <= tile)
+                for (int c = (i / SB + 1) * SB + 2 * lane; c < PB; c += 64)
                 {
-                    base += 2 * mi + 2;
-                    ++mi;
+                    out.pair(i, c, 0.0, 0.0);
                 }
-                const int ni = tile - base;
-                const int m0 = r0 + 16 * mi, n0 = r0 + 8 * ni;
-                double *c = sa + (m0 + g) * PS + n0 + 2 * t;
-                double cf[4] = { c[0], c[1], c[8 * PS], c[8 * PS + 1] };
-#pragma unroll
-                for (int kk = 0; kk < 4; ++kk)
+            }
+        }
+        else if (mover)
+        {
+            write_xs(s - 1, true, move_t, 32 * MOVE_WARPS);
+            bar_sync(SIDE_BAR, 32 * SIDE_WARPS);
+            // L's rows of sub-block s left of its diagonal
+            if (write_l)
+            {
+#pragma unroll 4
+                for (int i = c0 + move_w; i < c0 + SB; i += MOVE_WARPS)
                 {
-                    double af[4], bf[2];
-                    frag_a(af, sa, PS, m0, c0 + 8 * kk, g, t);
-                    frag_bt(bf, sa, PS, n0, c0 + 8 * kk, g, t);
 #pragma unroll
-                    for (int e = 0; e < 4; ++e)
+                    for (int c = 2 * lane; c < 3 * SB; c += 64)
                     {
-                        af[e] = -af[e];
+                        if (i < bs && c < c0)
+                        {
+                            const double2 v = *reinterpret_cast<const double2 *>(sa + i * PS + c);
+                            store_pair(A, lda, i, c, c0 - 1, al, v.x, v.y);
+                        }
                     }
-                    dmma(cf, af, bf);
                 }
-                c[0] = cf[0];
-                c[1] = cf[1];
-                c[8 * PS] = cf[2];
-                c[8 * PS + 1] = cf[3];
-            }
-        }
-        __syncthreads();
-    }
-    if (tid == 0 && bad != 0 && status != nullptr)
-    {
-        atomicCAS(&status->not_spd_row, 0, bad);
-    }
-    assemble_row_block(sa, xall + 3 * SB * XS, tbuf, 3, 0, NWARPS, 0);
-    __syncthreads();
-    pdl_launch_dependents();  // only the stores are left
-    // store Linv (zero above the diagonal) in pairs of columns
-#pragma unroll 8
-    for (int q = 0; q < PB * PB / 2 / PTHREADS; ++q)
-    {
-        const int idx = q * PTHREADS + tid;
-        const int i = idx >> 6, c = 2 * (idx & 63);
-        if (i >= bs || c >= bs)
-        {
-            continue;
-        }
-        const double2 raw = *reinterpret_cast<const double2 *>(sa + i * PS + c);
-        const double v0 = (c <= i) ? raw.x : 0.0;
-        const double v1 = (c + 1 <= i) ? raw.y : 0.0;
-        double *drow = (Linv != nullptr) ? Linv + static_cast<int64_t>(i) * ldi + c : nullptr;
-        float *frow = (Linv32 != nullptr) ? Linv32 + static_cast<int64_t>(i) * ldi32 + c : nullptr;
-        if (c + 1 < bs)
-        {
-            if (drow != nullptr)
-            {
-                *reinterpret_cast<double2 *>(drow) = make_double2(v0, v1);
-            }
-            if (frow != nullptr)
-            {
-                *reinterpret_cast<float2 *>(frow) = make_float2(static_cast<float>(v0), static_cast<float>(v1));
             }
         }
         else
         {
-            if (drow != nullptr)
+            // the rest of step s - 1
+            const int p = s - 1, p0 = p * SB;
+            const double *xp = xall + p * SB * XS;
+            const int b0 = c0 + SB;  // first row below the chain's sub-block
+            if (mma_w == 0)
             {
-                drow[0] = v0;
+                trailing_tile(sa, c0 + HB, c0 + HB, p0, g, t);
+                bar_arrive(HALF_BAR, 64);
             }
-            if (frow != nullptr)
+            // panel rows b0 ..: P = A X_p^T, in place, a warp takes 16 rows
+            for (int m0 = b0 + 16 * (mma_w - 1); m0 < PB && mma_w > 0; m0 += 16 * MMA_WARPS)
             {
-                frow[0] = static_cast<float>(v0);
+                double af[4][4];
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk)
+                {
+                    frag_a(af[kk], sa, PS, m0, p0 + 8 * kk, g, t);
+                }
+                __syncwarp();
+#pragma unroll
+                for (int nt = 0; nt < 4; ++nt)
+                {
+                    double cf[4] = { 0.0, 0.0, 0.0, 0.0 };
+#pragma unroll
+                    for (int kk = 0; kk <= nt; ++kk)  // X^T is zero where k > n
+                    {
+                        double bf[2];
+                        frag_bt(bf, xp, XS, 8 * nt, 8 * kk, g, t);
+                        dmma(cf, af[kk], bf);
+                    }
+                    const double r0 = rsq[p0 + 8 * nt + 2 * t], r1 = rsq[p0 + 8 * nt + 2 * t + 1];
+                    cf[0] *= r0;
+                    cf[1] *= r1;
+                    cf[2] *= r0;
+                    cf[3] *= r1;
+                    store_tile(sa, PS, m0, p0 + 8 * nt, cf, g, t);
+                }
             }
+            // row block p of the inverse, from the warps without panel rows on (5, 6, ..)
+            inverse_row_block(out, sa, true, xp, rsq, tbuf, p, (mma_w + MMA_WARPS - 5) % MMA_WARPS, MMA_WARPS, g, t);
+            bar_sync(SIDE_BAR, 32 * SIDE_WARPS);
+            // trailing update A -= P P^T of rows b0 .., columns c0 .. up to the diagonal, 16 x 16 tiles
+            const int mt = (PB - b0) / 16;
+            const int ntiles = mt * (mt + 5) / 2;  // sum over mi < mt of mi + 3
+            for (int tile = mma_w; tile < ntiles; tile += MMA_WARPS)
+            {
+                int mi = 0, base = 0;
+                while (base + mi + 3 <= tile)
+                {
+                    base += mi + 3;
+                    ++mi;
+                }
+                const int m0 = b0 + 16 * mi, n0 = c0 + 16 * (tile - base);
+                trailing_tile(sa, m0, n0, p0, g, t);
+            }
+            inverse_temporary(tbuf, sa, s, MMA_WARPS - 1 - mma_w, MMA_WARPS, g, t);
+            write_diag(p, 32 * mma_w + lane, 32 * MMA_WARPS);
         }
+        if (s == 0)
+        {
+            asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        }
+        __syncthreads();
+        if (s == 3)
+        {
+            if (warp == 0)
+            {
+                finish_pivots(3);
+            }
+            __syncthreads();
+            break;
+        }
+        // what the next chain waits for.  Panel rows of sub-block s+1: eight warps
+        // take one 16 x 8 tile each (every scheduler the same number of products:
+        // X^T is zero where k > n); all read before any writes.
+        const int c1 = c0 + SB;
+        const int mi = warp >> 2, nt = mi == 0 ? warp & 3 : 3 - (warp & 3);
+        double af[4][4], bf[4][2], cf[4] = {};
+        if (warp < 8)
+        {
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk)
+            {
+                if (kk <= nt)
+                {
+                    frag_a(af[kk], sa, PS, c1 + 16 * mi, c0 + 8 * kk, g, t);
+                    frag_bt(bf[kk], xs, XS, 8 * nt, 8 * kk, g, t);
+                    dmma(cf, af[kk], bf[kk]);
+                }
+            }
+            // the scaling of X's rows, beside the products
+            const double r0 = inv_sqrt(piv[c0 + 8 * nt + 2 * t]), r1 = inv_sqrt(piv[c0 + 8 * nt + 2 * t + 1]);
+            cf[0] *= r0;
+            cf[1] *= r1;
+            cf[2] *= r0;
+            cf[3] *= r1;
+        }
+        else if (warp == 8)
+        {
+            finish_pivots(s);
+        }
+        __syncthreads();
+        if (warp < 8)
+        {
+            store_tile(sa, PS, c1 + 16 * mi, c0 + 8 * nt, cf, g, t);
+        }
+        __syncthreads();
+        // the first 16 columns of its diagonal sub-block, one 16 x 8 tile per scheduler
+        if (warp < 4)
+        {
+            const int m0 = c1 + 16 * (warp >> 1), n0 = c1 + 8 * (warp & 1);
+            double ct[4] = {};
+            const double *c = sa + (m0 + g) * PS + n0 + 2 * t;
+            const double2 v0 = *reinterpret_cast<const double2 *>(c);
+            const double2 v1 = *reinterpret_cast<const double2 *>(c + 8 * PS);
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk)
+            {
+                frag_a(af[kk], sa, PS, m0, c0 + 8 * kk, g, t);
+                frag_bt(bf[kk], sa, PS, n0, c0 + 8 * kk, g, t);
+            }
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk)
+            {
+                dmma(ct, af[kk], bf[kk]);
+            }
+            const double tile[4] = { v0.x - ct[0], v0.y - ct[1], v1.x - ct[2], v1.y - ct[3] };
+            store_tile(sa, PS, m0, n0, tile, g, t);
+        }
+        __syncthreads();
     }
+    pdl_launch_dependents();  // little more than the stores is left
+    if (tid == 0 && bad != 0 && status != nullptr)
+    {
+        atomicCAS(&status->not_spd_row, 0, bad);
+    }
+    inverse_row_block(out, sa, false, xall + 3 * SB * XS, rsq, tbuf, 3, warp, NWARPS, g, t);
+    write_xs(3, false, tid, PTHREADS);
+    write_diag(3, tid, PTHREADS);
 }
 
 }  // namespace
