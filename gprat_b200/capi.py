@@ -85,6 +85,10 @@ def _load() -> ctypes.CDLL:
     _vp, _i64p = ctypes.c_void_p, ctypes.POINTER(ctypes.c_int64)
     lib.gprat_cu_steps_enable.argtypes = [ctypes.c_int]
     lib.gprat_cu_test_trsv.argtypes = [ctypes.c_int, ctypes.c_int, _dp, _dp, _dp, _dp, ctypes.c_int]
+    lib.gprat_cu_test_dgemm_update.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int, _dp, _dp, _dp,
+                                               _dp, _dp, ctypes.c_int, _dp, _dp, ctypes.c_int]
+    lib.gprat_cu_test_dgemm_solve.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_int, _dp, _dp, _dp, _dp, _dp,
+                                              ctypes.c_int]
     lib.gprat_cu_test_set_wait_budget.argtypes = [_i64]
     _i8p, _i32p = ctypes.POINTER(ctypes.c_int8), ctypes.POINTER(ctypes.c_int32)
     lib.gprat_cu_test_oz_split.argtypes = [ctypes.c_int, ctypes.c_int, _dp, ctypes.c_int, ctypes.c_int, _i8p, _i32p]
@@ -197,6 +201,25 @@ def test_tc_gemm(kind: int, A: np.ndarray, B: np.ndarray, C: np.ndarray, alpha: 
     check(lib.gprat_cu_test_tc_gemm(int(kind), M, N, K, A.ctypes.data_as(_fp), K, B.ctypes.data_as(_fp), K,
                                     C.ctypes.data_as(_fp), C.shape[1], float(alpha), float(beta), int(bool(lower)),
                                     rp, int(tile_mode)))
+
+
+def test_dgemm_update(A0: np.ndarray, A1: np.ndarray, B: np.ndarray, C0: np.ndarray, C1: np.ndarray,
+                      lower: bool = False, z: Optional[np.ndarray] = None, y: Optional[np.ndarray] = None,
+                      tile: int = 0) -> None:
+    """Runs the FP64 update in place: C0 -= A0 B^T (lower: j <= i only), C1 -= A1 B^T, y -= B z
+    (C-contiguous float64; A0 or A1 may have no rows; tile 0 = automatic, 1 = 64x64, 2 = 32x32)."""
+    check(lib.gprat_cu_test_dgemm_update(A0.shape[0], A1.shape[0], B.shape[0], B.shape[1], _p(A0), _p(A1), _p(B),
+                                         _p(C0), _p(C1), int(bool(lower)), _p(z) if z is not None else None,
+                                         _p(y) if y is not None else None, int(tile)))
+
+
+def test_dgemm_solve(P0: np.ndarray, P1: np.ndarray, Linv: np.ndarray, rowsq: Optional[np.ndarray] = None,
+                     y: Optional[np.ndarray] = None, tile: int = 0) -> None:
+    """Runs the FP64 panel solve in place: P0, P1 := P Linv^T, rowsq += the rows' sums of squares of P1,
+    y := Linv y (C-contiguous float64; tile 0 = automatic, 1, 2, 4 = 16, 32, 64 rows per CTA)."""
+    check(lib.gprat_cu_test_dgemm_solve(P0.shape[0], P1.shape[0], Linv.shape[0], _p(P0), _p(P1), _p(Linv),
+                                        _p(rowsq) if rowsq is not None else None,
+                                        _p(y) if y is not None else None, int(tile)))
 
 
 def test_trsv(kind: int, L: np.ndarray, b: np.ndarray, max_ctas: int = 0) -> Tuple[np.ndarray, np.ndarray]:

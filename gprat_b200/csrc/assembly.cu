@@ -334,7 +334,7 @@ constexpr int MV_WARPS = 8;
 
 __global__ void __launch_bounds__(32 * MV_WARPS) cross_mv_kernel(const double *__restrict__ Kx, int64_t ldx, int m,
                                                                  int n, const double *__restrict__ alpha,
-                                                                 double *__restrict__ mean)
+                                                                 double *__restrict__ mean, int upper)
 {
     const int r = blockIdx.x * MV_WARPS + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
@@ -345,7 +345,7 @@ __global__ void __launch_bounds__(32 * MV_WARPS) cross_mv_kernel(const double *_
     const double *row = Kx + static_cast<int64_t>(r) * ldx;
     double s = 0.0;
     const int n2 = n & ~1;
-    for (int c = 2 * lane; c < n2; c += 64)
+    for (int c = (upper ? r & ~63 : 0) + 2 * lane; c < n2; c += 64)
     {
         const double2 k = *reinterpret_cast<const double2 *>(row + c);
         const double2 a = *reinterpret_cast<const double2 *>(alpha + c);
@@ -367,7 +367,8 @@ __global__ void __launch_bounds__(32 * MV_WARPS) cross_mv_kernel(const double *_
 }
 }  // namespace
 
-void cross_times_alpha(const double *Kx, int64_t ldx, int m, int n, const double *alpha, double *mean, cudaStream_t s)
+void cross_times_alpha(const double *Kx, int64_t ldx, int m, int n, const double *alpha, double *mean, cudaStream_t s,
+                       bool upper)
 {
     if (m <= 0)
     {
@@ -377,7 +378,7 @@ void cross_times_alpha(const double *Kx, int64_t ldx, int m, int n, const double
     {
         throw Error(1, "cross_times_alpha: Kx and alpha must be 16-byte aligned with an even leading dimension");
     }
-    cross_mv_kernel<<<ceil_div(m, MV_WARPS), 32 * MV_WARPS, 0, s>>>(Kx, ldx, m, n, alpha, mean);
+    cross_mv_kernel<<<ceil_div(m, MV_WARPS), 32 * MV_WARPS, 0, s>>>(Kx, ldx, m, n, alpha, mean, upper ? 1 : 0);
     GPRAT_LAUNCH_CHECK();
 }
 

@@ -152,29 +152,49 @@ inline int ceil_div(int64_t a, int64_t b) { return static_cast<int>((a + b - 1) 
 // Kernel launchers (defined in the .cu files).  All matrices are row-major
 // FP64 with an even leading dimension and 16-byte aligned bases.
 
-// C[MxN] = beta*C + alpha*op(A)*op(B) on FP64 DMMA tensor cores.
-//   transA=false: A is M x K (A[m*lda+k]); true: A stored K x M (A[k*lda+m]).
-//   transB=false: B stored K x N (B[k*ldb+n]); true: B stored N x K (B[n*ldb+k]).
-//   lower: M == N and only C[i][j] with i >= j is written (tiles above the
-//          diagonal are skipped).
-//   rowsq (optional, requires N <= 128): rowsq[i] += sum_j C_new[i][j]^2.
-struct GemmArgs
+// Rows of a product on the FP64 DMMA tensor cores: A (M x K, lda) and C (M x N, ldc).
+struct RowGroup
 {
-    int M, N, K;
     const double *A;
     int64_t lda;
-    bool transA;
-    const double *B;
-    int64_t ldb;
-    bool transB;
     double *C;
     int64_t ldc;
-    double alpha, beta;
-    bool lower;
-    double *rowsq;
-    int k_tri;  // if >0: for C row-tile starting at row r0, the K loop starts at r0 rounded down to k_tri (A upper-triangular-by-blocks)
+    int M;  // 0: no such rows
 };
-void dgemm(const GemmArgs &a, cudaStream_t s);
+
+// C -= A B^T (dgemm.cu) for up to two row groups that share B (N x K, ldb), in
+// one launch.  lower: of group 0 only C[i][j] with j <= i is written (M >= N).
+// y (optional): y -= B z as well (N and K values).
+struct UpdateArgs
+{
+    RowGroup rows[2];
+    const double *B;
+    int64_t ldb;
+    int N, K;
+    bool lower;
+    const double *z;
+    double *y;
+    bool c_first;          // subtract the products from C one by one instead of their sum
+    DeviceStatus *status;  // timeout flag of the bounded waits (may be null)
+    int tile;              // 0: by size (tests: 1 = 64 x 64 tiles, 2 = 32 x 32)
+};
+void dgemm_update(const UpdateArgs &a, cudaStream_t s);
+
+// P := P Linv^T in place for up to two row groups (A == C, bs <= 128 columns)
+// with one lower-triangular Linv (bs x bs, ldi).  rowsq (optional): of group 1,
+// rowsq[i] += sum_j P_new[i][j]^2.  y (optional): y := Linv y (bs values).
+struct SolveArgs
+{
+    RowGroup rows[2];
+    const double *Linv;
+    int64_t ldi;
+    int bs;
+    double *rowsq;
+    double *y;
+    DeviceStatus *status;
+    int tile;  // 0: by size (tests: 1, 2, 4 times 16 rows per CTA)
+};
+void dgemm_solve(const SolveArgs &a, cudaStream_t s);
 
 // SE covariance assembly (gen_tile_covariance, core/src/cpu/gp_algorithms.cpp:30-62):
 // K[i][j] = v*exp(-0.5/l^2 * sum_k (x[i+k]-x[j+k])^2) (+ noise if i == j), for all
@@ -199,8 +219,10 @@ void assemble_cross_f32(const double *xt, int m, const double *x, int n, int n_r
 // Cross covariance in FP64 (Kx, ldx) and its FP32 twin (Kx32, ld32) in one pass.
 void assemble_cross_dual(const double *xt, int m, const double *x, int n, int n_reg, const DeviceParams *p,
                          double *Kx, int64_t ldx, float *Kx32, int64_t ld32, cudaStream_t s);
-// mean = Kx alpha (m rows of Kx, n columns; deterministic).
-void cross_times_alpha(const double *Kx, int64_t ldx, int m, int n, const double *alpha, double *mean, cudaStream_t s);
+// mean = Kx alpha (m rows of Kx, n columns; deterministic).  upper: row r of Kx
+// is zero left of column r (not read).
+void cross_times_alpha(const double *Kx, int64_t ldx, int m, int n, const double *alpha, double *mean, cudaStream_t s,
+                       bool upper = false);
 void reduce_mean(const double *mean_partial, int m, int parts, double *mean, cudaStream_t s);
 
 // Prior covariance matrix K**[r][c] = k(xt_r, xt_c) (gen_tile_full_prior_covariance,
@@ -243,9 +265,12 @@ void trsv_fused_forward_f32(const float *L, int64_t ld, const float *Linv, int n
 void trsv_fused_backward_f32(const float *L, int64_t ld, const float *Linv, int n, double *x, int *flags,
                              double *scratch, DeviceStatus *st, cudaStream_t s, int max_ctas = 0,
                              const int *skip = nullptr);
-// Poll budget of the single-launch solves' waits on the current device
-// (polls < 0: the default, about 0.5-1 s).
-void set_trsv_wait_budget(long long polls);
+// Poll budget of the bounded waits on the current device: the single-launch
+// solves' on an unsolved block and the FP64 products' on their operand copies
+// (polls < 0: the defaults, about 0.5-1 s and 2 s).
+void set_wait_budget(long long polls);
+// The budget on the current device as the products take it (-1: the default).
+int wait_polls();
 // Same with an FP32 factor (mixed precision); FP64 right-hand side and arithmetic.
 void trsv_forward_f32(const float *L, int64_t ldl, const double *Linv, int nb, int n, double *rhs, cudaStream_t s);
 void trsv_backward_f32(const float *L, int64_t ldl, const double *Linv, int nb, int n, double *rhs, cudaStream_t s);
@@ -262,10 +287,11 @@ void finalize_variance(const double *acc, int m, const DeviceParams *p, double *
 void set_identity(double *A, int64_t lda, int n, cudaStream_t s);
 void copy_rows(const double *src, int64_t lds, double *dst, int64_t ldd, int rows, int cols, cudaStream_t s);
 
-// Adjoint: per lower tile partial sums of (Kinv - a a^T) .* dK for l and v, and
+// Adjoint (U: 16-byte aligned, even ldu): per lower tile partial sums of (Kinv - a a^T) .* dK for l and v, and
 // the noise term; then reduction + Adam (see optimizer.cu).
 void adjoint_trace(const double *U, int64_t ldu, const double *alpha, const double *x, int n, int n_reg,
-                   const DeviceParams *p, double *partials, int *n_partials, cudaStream_t s);
+                   const DeviceParams *p, double *partials, int *n_partials, DeviceStatus *status,
+                   cudaStream_t s);
 void adjoint_finish(const double *partials, int n_partials, int n, DeviceParams *p, bool adam_step,
                     cudaStream_t s);
 

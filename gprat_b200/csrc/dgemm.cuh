@@ -1,155 +1,316 @@
-// FP64 tensor-core (DMMA, mma.sync m16n8k8 .f64) GEMM mainloop for sm_100a.
+// FP64 tensor-core (DMMA, mma.sync m16n8k8 .f64) building blocks on sm_100a:
+// the TMA-fed main loop shared by the updates (dgemm.cu) and the adjoint
+// kernel (optimizer.cu).
 //
-// Two CTA shapes share one mainloop (template parameter WN = warps along N):
-//   WN = 4: CTA tile 128x128, 8 warps, 4-stage pipeline, 1 CTA/SM.  Used
-//           when N <= 128 (panel solves, in-place diagonal-block steps).
-//   WN = 2: CTA tile 128x64, 4 warps, 3-stage pipeline, 2 CTAs/SM, so one
-//           CTA's C load/store overlaps the other CTA's DMMA main loop.
-//           Used for the large trailing updates.
-// Warp tile 64x32 = 4x4 m16n8k8 fragments (64 FP64 accumulators/thread).
-// K step 16 via cp.async.  Shared-memory rows are padded so every fragment
-// load is conflict-free (row stride = 4 mod 16 doubles when K is the
-// contiguous index, 8 mod 16 when M/N is).  The epilogue is supplied by the
-// kernel that instantiates the mainloop.
+// DMMA and the FP64 FMA units have the same peak here (128 flops per cycle and
+// SM, 37.2 TFLOP/s), and one warp per scheduler with 16 independent products
+// reaches 98 % of it (65.4 cycles per product instead of 64), so a main loop is
+// as good as the time its warps are not stalled on anything else:
+//   * a group of four warps (2 x 2) owns a C tile of 32 FM x 16 FN, a warp
+//     FM x FN fragments of 16 x 8; no barrier inside the group: every warp
+//     waits on the stage's full barrier and releases the stage by itself;
+//   * the operand ring is filled by TMA copies, one per operand and stage;
+//   * three CTAs of one 64 x 64 tile share an SM, so one's start and write-out
+//     lie under the others' products (two groups of one persistent CTA with
+//     128 x 64 tiles, which run in step, reach 29 TFLOP/s where this reaches
+//     33.8, at 8192 x 8192 x 512);
+//   * operand boxes are 8 columns (64 bytes) wide, and a thread takes columns
+//     2t and 2t + 1 as the product's k = t and k = t + 4 (the order of k is free
+//     as long as A and B agree): one 16-byte shared load per fragment row, and
+//     eight lanes of a quarter warp read 128 contiguous bytes, so no bank
+//     conflicts without padding or swizzle;
+//   * the fragments of the next k step are loaded while the current one's
+//     products are in the pipe.
+// A copy fills what lies outside an operand with zeros, so ragged K needs no
+// special case.  Waits are bounded: one that runs out raises the CTA's abort
+// flag, later waits return at once, and the status word's timeout flag makes
+// the host call fail.
 #pragma once
 
 #include "common.cuh"
-
-#include <type_traits>
+#include "tcgen05_ptx.cuh"
 
 namespace gprat_cu
 {
 namespace gemm
 {
 
-#ifndef GPRAT_DGEMM_BK
-#define GPRAT_DGEMM_BK 16
-#endif
-constexpr int BK = GPRAT_DGEMM_BK;  // K per pipeline stage
-constexpr int PAD_K = 4;  // stride BK+4 doubles (conflict-free fragment loads)
-constexpr int PAD_T = 8;  // stride ROWS+8 doubles
+constexpr int KC = 8;      // columns of a TMA box (64 bytes)
+constexpr int BK = 2 * KC;  // K per stage
+constexpr int STAGES = 4;
+constexpr int GROUP_THREADS = 128;
 
-template <int WN>
-struct Cfg
+template <int FM, int FN>
+struct Tile
 {
-    static constexpr int WM = 2;
-    static constexpr int THREADS = 32 * WM * WN;
-    static constexpr int BM = 64 * WM;  // 128
-    static constexpr int BN = 32 * WN;  // 128 or 64
-    static constexpr int STAGES = (WN == 4) ? (BK == 16 ? 4 : 3) : (BK == 16 ? 3 : 2);
-    static constexpr int MIN_BLOCKS = (WN == 4) ? 1 : 2;
+    static constexpr int BM = 32 * FM;
+    static constexpr int BN = 16 * FN;
+    static constexpr int A_DOUBLES = BM * BK;
+    static constexpr int STAGE_DOUBLES = (BM + BN) * BK;
+    static constexpr int RING_BYTES = STAGES * STAGE_DOUBLES * 8;
 };
 
-// Operand tile whose rows run along K: [ROWS][BK+PAD_K]
-template <int ROWS>
-struct KMajor
+// One tile of the stream a group works through: which A, where, and its K range.
+struct TileJob
 {
-    static constexpr int SIZE = ROWS * (BK + PAD_K);
-    __device__ __forceinline__ static int idx(int row, int k) { return row * (BK + PAD_K) + k; }
+    int a;       // row group: which A operand (and C)
+    int m0, n0;  // rows of A, rows of B
+    int k0, k1;
 };
 
-// Operand tile whose rows run along M or N: [BK][ROWS+PAD_T]
-template <int ROWS>
-struct RMajor
+// Barriers of one group's ring.
+struct RingBars
 {
-    static constexpr int SIZE = BK * (ROWS + PAD_T);
-    __device__ __forceinline__ static int idx(int row, int k) { return k * (ROWS + PAD_T) + row; }
+    uint64_t full[STAGES];
+    uint64_t empty[STAGES];
 };
 
-// A: transA=false -> A[m][k] rows along K -> KMajor; true -> RMajor.
-// B: transB=true  -> B[n][k] rows along K -> KMajor; false -> RMajor.
-template <bool TA, int ROWS>
-using ALayout = typename std::conditional<TA, RMajor<ROWS>, KMajor<ROWS>>::type;
-template <bool TB, int ROWS>
-using BLayout = typename std::conditional<TB, KMajor<ROWS>, RMajor<ROWS>>::type;
-
-template <int WN, bool TA, bool TB>
-constexpr int smem_bytes()
+__device__ __forceinline__ void init_ring(RingBars &bars)
 {
-    using C = Cfg<WN>;
-    return C::STAGES * (ALayout<TA, C::BM>::SIZE + BLayout<TB, C::BN>::SIZE) * 8;
+    for (int st = 0; st < STAGES; ++st)
+    {
+        tcx::mbar_init(&bars.full[st], 1);
+        tcx::mbar_init(&bars.empty[st], 4);
+    }
 }
 
-__device__ __forceinline__ void cp_async16(void *smem, const void *gmem, int src_bytes)
+// Bounded wait for a barrier's phase: polls times where polls >= 0 (a test's
+// budget), else about two seconds.  False: it gave up, now or before (the abort
+// flag); a thread that sees false issues no further copy.
+__device__ __forceinline__ bool ring_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag, int polls)
 {
-    unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(src_bytes));
-}
-
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
-
-template <int N>
-__device__ __forceinline__ void cp_async_wait()
-{
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
+    if (tcx::mbar_test_wait(bar, parity))
+    {
+        return true;
+    }
+    if (polls < 0)
+    {
+        return tcx::mbar_wait(bar, parity, abort_flag);
+    }
+    for (int i = 0; i < polls; ++i)
+    {
+        if (*abort_flag != 0)
+        {
+            return false;
+        }
+        if (tcx::mbar_try_wait(bar, parity))
+        {
+            return true;
+        }
+    }
+    *abort_flag = 1;
+    return false;
 }
 
 __device__ __forceinline__ void dmma_16x8x8(double (&d)[4], const double (&a)[4], const double (&b)[2])
 {
-    asm volatile(
-        "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+    asm("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
         "{%0,%1,%2,%3};\n"
         : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
         : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
 }
 
-// Copies one operand tile (ROWS rows of the operand starting at r0, K range
-// [k0, k0+BK)) into shared memory with zero fill outside [rows) x [K).
-// KMAJOR: element (row, k) at P[row*ld + k]; otherwise at P[k*ld + row].
-template <bool KMAJOR, int ROWS, int THREADS>
-__device__ __forceinline__ void load_tile(double *s, const double *P, int64_t ld, int rows, int K, int r0, int k0,
-                                          int tid)
+__device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, int x, int y, uint64_t *bar)
 {
-    if (KMAJOR)
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+            tcx::smem_u32(dst)),
+        "l"(map), "r"(x), "r"(y), "r"(tcx::smem_u32(bar))
+        : "memory");
+}
+
+__device__ __forceinline__ void prefetch_map(const CUtensorMap *map)
+{
+    asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
+}
+
+__device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, int x, int y, int z, uint64_t *bar)
+{
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], "
+        "[%5];" ::"r"(tcx::smem_u32(dst)),
+        "l"(map), "r"(x), "r"(y), "r"(z), "r"(tcx::smem_u32(bar))
+        : "memory");
+}
+
+// An operand's tensor map: a matrix whose column count is a multiple of 8 as
+// (8 columns, rows, column groups), so that one copy brings a stage's two boxes
+// (`grouped`); any other as (columns, rows), one box per copy, whose fill of
+// zeros ends at the last column.
+// Columns k .. k + 15 of `rows` rows from `row`: two boxes.
+__device__ __forceinline__ void load_boxes(double *dst, const CUtensorMap *map, bool grouped, int k, int row, int rows,
+                                           uint64_t *bar)
+{
+    if (grouped)
     {
-        constexpr int CHUNKS = ROWS * (BK / 2);
-#pragma unroll
-        for (int i = 0; i < CHUNKS / THREADS; ++i)
-        {
-            int c = tid + i * THREADS;
-            int row = c / (BK / 2);
-            int kc = (c % (BK / 2)) * 2;
-            int gr = r0 + row, gk = k0 + kc;
-            int nv = (gr < rows) ? min(max(K - gk, 0), 2) : 0;
-            const double *src = nv ? P + static_cast<int64_t>(gr) * ld + gk : P;
-            cp_async16(s + KMajor<ROWS>::idx(row, kc), src, nv * 8);
-        }
+        tma_load_3d(dst, map, 0, row, k / KC, bar);
     }
     else
     {
-        constexpr int PER_ROW = ROWS / 2;
-        constexpr int CHUNKS = BK * PER_ROW;
+        tma_load_2d(dst, map, k, row, bar);
+        tma_load_2d(dst + rows * KC, map, k + KC, row, bar);
+    }
+}
+
+// A fragment row pair / B fragment row: two columns per thread.
+template <int FM>
+__device__ __forceinline__ void load_a(double (&a)[FM][4], const double *box, int row, int t)
+{
 #pragma unroll
-        for (int i = 0; i < CHUNKS / THREADS; ++i)
+    for (int mi = 0; mi < FM; ++mi)
+    {
+        const double2 u = *reinterpret_cast<const double2 *>(box + (row + 16 * mi) * KC + 2 * t);
+        const double2 v = *reinterpret_cast<const double2 *>(box + (row + 16 * mi + 8) * KC + 2 * t);
+        a[mi][0] = u.x;
+        a[mi][1] = v.x;
+        a[mi][2] = u.y;
+        a[mi][3] = v.y;
+    }
+}
+
+template <int FN>
+__device__ __forceinline__ void load_b(double (&b)[FN][2], const double *box, int row, int t)
+{
+#pragma unroll
+    for (int ni = 0; ni < FN; ++ni)
+    {
+        const double2 u = *reinterpret_cast<const double2 *>(box + (row + 8 * ni) * KC + 2 * t);
+        b[ni][0] = u.x;
+        b[ni][1] = u.y;
+    }
+}
+
+template <int FM, int FN>
+__device__ __forceinline__ void products(double (&acc)[FM][FN][4], const double (&a)[FM][4], const double (&b)[FN][2])
+{
+#pragma unroll
+    for (int mi = 0; mi < FM; ++mi)
+    {
+#pragma unroll
+        for (int ni = 0; ni < FN; ++ni)
         {
-            int c = tid + i * THREADS;
-            int krow = c / PER_ROW;
-            int rc = (c % PER_ROW) * 2;
-            int gk = k0 + krow, gr = r0 + rc;
-            int nv = (gk < K) ? min(max(rows - gr, 0), 2) : 0;
-            const double *src = nv ? P + static_cast<int64_t>(gk) * ld + gr : P;
-            cp_async16(s + RMajor<ROWS>::idx(rc, krow), src, nv * 8);
+            dmma_16x8x8(acc[mi][ni], a[mi], b[ni]);
         }
     }
 }
 
-struct TileCoord
+// The group's operand ring for one tile, as its producer (one thread) and its
+// four warps see it.
+template <int FM, int FN>
+struct Ring
 {
-    int m0, n0;
+    using T = Tile<FM, FN>;
+    double *ring;
+    RingBars *bars;
+    volatile int *abort_flag;
+    const CUtensorMap *map_a, *map_b;
+    bool grouped;
+    int polls;
+    TileJob job;
+
+    // producer: the copies of stage number `it` of the tile
+    __device__ __forceinline__ void load(int it) const
+    {
+        const int st = it % STAGES, k = job.k0 + it * BK;
+        double *dst = ring + st * T::STAGE_DOUBLES;
+        tcx::mbar_expect_tx(&bars->full[st], T::STAGE_DOUBLES * 8);
+        load_boxes(dst, map_a, grouped, k, job.m0, T::BM, &bars->full[st]);
+        load_boxes(dst + T::A_DOUBLES, map_b, grouped, k, job.n0, T::BN, &bars->full[st]);
+    }
+
+    __device__ __forceinline__ int stages() const { return (job.k1 - job.k0 + BK - 1) / BK; }
+
+    // one thread: the first stages
+    __device__ __forceinline__ void begin() const
+    {
+        if (threadIdx.x == 0)
+        {
+#pragma unroll 1
+            for (int q = 0; q < STAGES && q < stages(); ++q)
+            {
+                load(q);
+            }
+        }
+    }
+
+    // acc += A B^T over the tile's K range.  arow / brow: this thread's first
+    // fragment rows in the tile.  The warps take turns at refilling stages
+    // (issuing a copy costs a small tile's warp as much as its products).
+    __device__ __forceinline__ void run(double (&acc)[FM][FN][4], int arow, int brow, int t) const
+    {
+        const int nk = stages(), warp = threadIdx.x >> 5;
+        double a[2][FM][4], b[2][FN][2];
+        const double *box = ring;
+        ring_wait(&bars->full[0], 0, abort_flag, polls);
+        load_a(a[0], box, arow, t);
+        load_b(b[0], box + T::A_DOUBLES, brow, t);
+#pragma unroll 1
+        for (int kt = 0; kt < nk; ++kt)
+        {
+            load_a(a[1], box + T::BM * KC, arow, t);
+            load_b(b[1], box + T::A_DOUBLES + T::BN * KC, brow, t);
+            products(acc, a[0], b[0]);
+            __syncwarp();
+            if ((threadIdx.x & 31) == 0)
+            {
+                tcx::mbar_arrive(&bars->empty[kt % STAGES]);
+                const int next = kt - 1 + STAGES;  // refills the stage the group left one step ago
+                // (a warp that gave up arrives without having waited, so the flag is
+                // looked at after the wait: a stage is never loaded twice at once)
+                if (warp == (kt & 3) && kt > 0 && next < nk &&
+                    ring_wait(&bars->empty[(kt - 1) % STAGES], ((kt - 1) / STAGES) & 1, abort_flag, polls) &&
+                    *abort_flag == 0)
+                {
+                    load(next);
+                }
+            }
+            if (kt + 1 < nk)
+            {
+                const int st = (kt + 1) % STAGES;
+                box = ring + st * T::STAGE_DOUBLES;
+                ring_wait(&bars->full[st], ((kt + 1) / STAGES) & 1, abort_flag, polls);
+                load_a(a[0], box, arow, t);
+                load_b(b[0], box + T::A_DOUBLES, brow, t);
+            }
+            products(acc, a[1], b[1]);
+        }
+    }
 };
 
-// Maps blockIdx to the C tile.  In `lower` mode the grid is 1-D over the
-// tiles that touch the lower triangle: row tile i (BM high) has (i+1)*BM/BN
+// After a timeout: copies may still be in flight towards this CTA's shared
+// memory; they land long before this returns.
+__device__ __forceinline__ void drain_after_abort()
+{
+    const unsigned long long t0 = tcx::global_ns();
+    for (int i = 0; i < 100000 && tcx::global_ns() - t0 < 200000ull; ++i)
+    {
+        __nanosleep(1000);
+    }
+}
+
+// Row tiles of the lower trapezoid C[i][j], j <= i, of an M x N product (M >= N)
+// in BM x BN tiles, BM a multiple of BN: row tile i has min((i + 1) BM / BN, NT)
 // column tiles.
 template <int BM, int BN>
-__device__ __forceinline__ TileCoord tile_coord(bool lower)
+__host__ __device__ inline int trapezoid_tiles(int M, int N)
 {
-    TileCoord t;
-    if (lower)
+    constexpr int R = BM / BN;
+    const int mt = (M + BM - 1) / BM, nt = (N + BN - 1) / BN;
+    const int tri = mt < nt / R ? mt : nt / R;
+    return R * tri * (tri + 1) / 2 + (mt - tri) * nt;
+}
+
+template <int BM, int BN>
+__device__ __forceinline__ void trapezoid_tile(int q, int M, int N, int &m0, int &n0)
+{
+    constexpr int R = BM / BN;
+    const int mt = (M + BM - 1) / BM, nt = (N + BN - 1) / BN;
+    const int tri = mt < nt / R ? mt : nt / R;
+    const int first = R * tri * (tri + 1) / 2;
+    int i, j;
+    if (q < first)
     {
-        constexpr int R = BM / BN;
-        const int q = blockIdx.x;
-        int i = static_cast<int>((sqrt(8.0 * q / R + 1.0) - 1.0) * 0.5);
+        i = static_cast<int>((sqrtf(8.0f * static_cast<float>(q) / R + 1.0f) - 1.0f) * 0.5f);
         while (R * (i + 1) * (i + 2) / 2 <= q)
         {
             ++i;
@@ -158,124 +319,22 @@ __device__ __forceinline__ TileCoord tile_coord(bool lower)
         {
             --i;
         }
-        t.m0 = i * BM;
-        t.n0 = (q - R * i * (i + 1) / 2) * BN;
+        j = q - R * i * (i + 1) / 2;
     }
     else
     {
-        t.m0 = blockIdx.y * BM;
-        t.n0 = blockIdx.x * BN;
+        i = tri + (q - first) / nt;
+        j = (q - first) % nt;
     }
-    return t;
+    m0 = i * BM;
+    n0 = j * BN;
 }
 
-template <int BM, int BN>
-inline int lower_grid(int M)
-{
-    const int t = (M + BM - 1) / BM;
-    return (BM / BN) * t * (t + 1) / 2;
-}
-
-// acc[mi][ni][0..3]: rows wm*64+mi*16+g (+8 for [2],[3]), cols wn*32+ni*8+2t (+1)
-struct Frag
-{
-    int g, t, wm, wn;
-};
-
-template <int WN>
-__device__ __forceinline__ Frag frag_coords()
-{
-    Frag f;
-    int lane = threadIdx.x & 31;
-    int warp = threadIdx.x >> 5;
-    f.g = lane >> 2;
-    f.t = lane & 3;
-    f.wm = warp / WN;  // 0..1
-    f.wn = warp % WN;
-    return f;
-}
-
-template <int WN, bool TA, bool TB>
-__device__ __forceinline__ void mainloop(const GemmArgs &a, int m0, int n0, double *smem, double (&acc)[4][4][4],
-                                         int k_begin, const Frag &f)
-{
-    using C = Cfg<WN>;
-    using LA = ALayout<TA, C::BM>;
-    using LB = BLayout<TB, C::BN>;
-    constexpr int STAGES = C::STAGES;
-    double *sA = smem;
-    double *sB = smem + STAGES * LA::SIZE;
-    const int tid = threadIdx.x;
-    const int kspan = a.K - k_begin;
-    const int KT = kspan > 0 ? (kspan + BK - 1) / BK : 0;
-
-    auto load_stage = [&](int kt, int stage)
-    {
-        int k0 = k_begin + kt * BK;
-        load_tile<!TA, C::BM, C::THREADS>(sA + stage * LA::SIZE, a.A, a.lda, a.M, a.K, m0, k0, tid);
-        load_tile<TB, C::BN, C::THREADS>(sB + stage * LB::SIZE, a.B, a.ldb, a.N, a.K, n0, k0, tid);
-    };
-
-#pragma unroll
-    for (int s = 0; s < STAGES - 1; ++s)
-    {
-        if (s < KT)
-        {
-            load_stage(s, s);
-        }
-        cp_async_commit();
-    }
-
-    for (int kt = 0; kt < KT; ++kt)
-    {
-        cp_async_wait<STAGES - 2>();
-        __syncthreads();
-        int nk = kt + STAGES - 1;
-        if (nk < KT)
-        {
-            load_stage(nk, nk % STAGES);
-        }
-        cp_async_commit();
-
-        const double *cA = sA + (kt % STAGES) * LA::SIZE;
-        const double *cB = sB + (kt % STAGES) * LB::SIZE;
-#pragma unroll
-        for (int ks = 0; ks < BK / 8; ++ks)
-        {
-            double af[4][4];
-            double bf[4][2];
-#pragma unroll
-            for (int mi = 0; mi < 4; ++mi)
-            {
-                int r = f.wm * 64 + mi * 16 + f.g;
-                int c = ks * 8 + f.t;
-                af[mi][0] = cA[LA::idx(r, c)];
-                af[mi][1] = cA[LA::idx(r + 8, c)];
-                af[mi][2] = cA[LA::idx(r, c + 4)];
-                af[mi][3] = cA[LA::idx(r + 8, c + 4)];
-            }
-#pragma unroll
-            for (int ni = 0; ni < 4; ++ni)
-            {
-                int n = f.wn * 32 + ni * 8 + f.g;
-                int k = ks * 8 + f.t;
-                bf[ni][0] = cB[LB::idx(n, k)];
-                bf[ni][1] = cB[LB::idx(n, k + 4)];
-            }
-#pragma unroll
-            for (int mi = 0; mi < 4; ++mi)
-            {
-#pragma unroll
-                for (int ni = 0; ni < 4; ++ni)
-                {
-                    dmma_16x8x8(acc[mi][ni], af[mi], bf[ni]);
-                }
-            }
-        }
-    }
-    cp_async_wait<0>();
-    __syncthreads();
-}
+// Tensor map of a row-major FP64 matrix (rows x cols, ld) for load_boxes
+// (dgemm.cu).
+void make_map(CUtensorMap &map, const double *base, int rows, int cols, int64_t ld, int box_rows);
+// Whether a matrix with that many columns gets a grouped map.
+constexpr bool grouped_map(int cols) { return cols % KC == 0; }
 
 }  // namespace gemm
 }  // namespace gprat_cu

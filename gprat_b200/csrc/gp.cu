@@ -7,16 +7,16 @@
 // n_test x n solve matrix, the inverse factor for the optimiser).
 //
 // Pipelines (reference files in parentheses, relative to the project root):
-//   factor   = SE assembly of the lower tiles + blocked right-looking
-//              Cholesky: potrf+inverse of the diagonal block, panel solve as
-//              a DMMA GEMM with the inverse, lower-only DMMA trailing update
-//              (right_looking_cholesky_tiled, core/src/cpu/tiled_algorithms.cpp:14-57)
-//   alpha    = blocked forward/backward solves (:61-115)
-//   mean     = cross covariance fused with the mat-vec (:187-210)
-//   variance = right-looking solve W L^T = K*  with the row sums of W^2
-//              fused into the diagonal-block step (:117-149, :212-263)
+//   factor   = SE assembly of the lower tiles + blocked Cholesky (fp64_path.cu:
+//              right_looking_cholesky_tiled, core/src/cpu/tiled_algorithms.cpp:14-57)
+//   alpha    = forward solve along with the factorisation, backward solve in
+//              one kernel (:61-115)
+//   mean     = cross covariance fused with the mat-vec (:187-210), or with the
+//              variance W (L^-1 y)
+//   variance = W L^T = K*, with the factorisation, row sums of W^2 fused into
+//              the panel solves (:117-149, :212-263)
 //   loss     = (core/src/cpu/gp_optimizer.cpp:187-218)
-//   gradient = U = L^-T, fused K^-1 = U U^T tile GEMM + derivative-tile
+//   gradient = U = L^-T with the factorisation, fused K^-1 = U U^T tile GEMM + derivative-tile
 //              regeneration + trace reduction, then Adam (optimizer.cu)
 #include "common.cuh"
 #include "gp_state.cuh"
@@ -117,94 +117,24 @@ void upload_hyper(gprat_cu_gp *gp, const double hyper[3], cudaStream_t s)
     GPRAT_CUDA_CHECK(cudaMemsetAsync(gp->status.ptr, 0, sizeof(DeviceStatus), s));
 }
 
-double *kblock(gprat_cu_gp *gp, int r, int c) { return gp->K.ptr + static_cast<int64_t>(r) * gp->ld + c; }
-
-double *linv_block(gprat_cu_gp *gp, int k) { return gp->Linv.ptr + static_cast<int64_t>(k) * NB * NB; }
-
-// C[MxN] = beta*C + alpha * A B^T (A: M x K, B: N x K, row-major)
-void gemm_nt(int M, int N, int K, const double *A, int64_t lda, const double *B, int64_t ldb, double *C,
-             int64_t ldc, double alpha, double beta, bool lower, double *rowsq, cudaStream_t s)
-{
-    GemmArgs g{};
-    g.M = M;
-    g.N = N;
-    g.K = K;
-    g.A = A;
-    g.lda = lda;
-    g.transA = false;
-    g.B = B;
-    g.ldb = ldb;
-    g.transB = true;
-    g.C = C;
-    g.ldc = ldc;
-    g.alpha = alpha;
-    g.beta = beta;
-    g.lower = lower;
-    g.rowsq = rowsq;
-    dgemm(g, s);
-}
-
-// Two-level right-looking blocked Cholesky.  Inner steps (NB = 128): FP64
-// potrf + inverse of the diagonal block, panel solve P = P Linv^T (in place),
-// and the update of the rest of the current outer panel.  Outer steps
-// (NBO = 512): one lower-triangular DMMA update of the trailing matrix with
-// K = 512.
-void cholesky_blocked(gprat_cu_gp *gp, cudaStream_t s)
-{
-    const int n = gp->n;
-    const int64_t ld = gp->ld;
-    for (int K0 = 0; K0 < n; K0 += NBO)
-    {
-        const int bo = std::min(NBO, n - K0);
-        const int pend = K0 + bo;  // end of this outer panel
-        for (int r0 = K0; r0 < pend; r0 += NB)
-        {
-            const int bs = std::min(NB, pend - r0);
-            const int k = r0 / NB;
-            potrf_diag(kblock(gp, r0, r0), ld, bs, r0, linv_block(gp, k), NB, gp->status.ptr, s);
-            const int rows = n - r0 - bs;
-            if (rows <= 0)
-            {
-                continue;
-            }
-            // panel solve: P = P * Linv_kk^T (in place; one CTA column since bs <= 128)
-            gemm_nt(rows, bs, bs, kblock(gp, r0 + bs, r0), ld, linv_block(gp, k), NB, kblock(gp, r0 + bs, r0), ld,
-                    1.0, 0.0, false, nullptr, s);
-            // update the rest of the outer panel: columns [r0+bs, pend)
-            const int ncols = pend - (r0 + bs);
-            if (ncols > 0)
-            {
-                // square part (rows [r0+bs, pend)): lower triangle only
-                gemm_nt(ncols, ncols, bs, kblock(gp, r0 + bs, r0), ld, kblock(gp, r0 + bs, r0), ld,
-                        kblock(gp, r0 + bs, r0 + bs), ld, -1.0, 1.0, true, nullptr, s);
-                // rows below the outer panel
-                const int below = n - pend;
-                if (below > 0)
-                {
-                    gemm_nt(below, ncols, bs, kblock(gp, pend, r0), ld, kblock(gp, r0 + bs, r0), ld,
-                            kblock(gp, pend, r0 + bs), ld, -1.0, 1.0, false, nullptr, s);
-                }
-            }
-        }
-        const int rest = n - pend;
-        if (rest > 0)
-        {
-            // outer trailing update: C -= P_o P_o^T, K = bo, lower triangle only
-            gemm_nt(rest, rest, bo, kblock(gp, pend, K0), ld, kblock(gp, pend, K0), ld, kblock(gp, pend, pend), ld,
-                    -1.0, 1.0, true, nullptr, s);
-        }
-    }
-}
-
-// FP64 factorisation (always used by cholesky() and the optimiser).
-void factor_fp64(gprat_cu_gp *gp, cudaStream_t s)
+// Covariance and FP64 factorisation (always used by cholesky() and the
+// optimiser), with e's rows and vector solved along.
+void factor_fp64(gprat_cu_gp *gp, const SolveRows &e, cudaStream_t s)
 {
     {
         StepScope step("assembly", s);
         assemble_covariance(gp->x.ptr, gp->n, gp->d, gp->T, gp->params.ptr, gp->K.ptr, gp->ld, s);
     }
-    StepScope step("cholesky", s);
-    cholesky_blocked(gp, s);
+    factor_solve_fp64(gp, e, s);
+}
+
+// The same with z = L^-1 y (gp->z).
+void factor_forward_fp64(gprat_cu_gp *gp, SolveRows e, cudaStream_t s)
+{
+    gp->z.ensure(gp->n);
+    GPRAT_CUDA_CHECK(cudaMemcpyAsync(gp->z.ptr, gp->y.ptr, gp->n * sizeof(double), cudaMemcpyDeviceToDevice, s));
+    e.vec = gp->z.ptr;
+    factor_fp64(gp, e, s);
 }
 
 // The TF32 / BF16 modes: a low-precision working copy of the factor, alpha
@@ -231,16 +161,27 @@ void fit(gprat_cu_gp *gp, cudaStream_t s)
         factor_oz(gp, s);
         solve_alpha_fp64(gp, s);
     }
+    else if (steps_enabled())
+    {
+        // step timers: the phases apart
+        factor_fp64(gp, SolveRows{}, s);
+        solve_alpha_fp64(gp, s);
+    }
     else
     {
-        factor_fp64(gp, s);
-        solve_alpha_fp64(gp, s);
+        factor_forward_fp64(gp, SolveRows{}, s);
+        gp->flags.ensure(2);
+        gp->trsv_b.ensure(gp->n);
+        GPRAT_CUDA_CHECK(
+            cudaMemcpyAsync(gp->alpha.ptr, gp->z.ptr, gp->n * sizeof(double), cudaMemcpyDeviceToDevice, s));
+        trsv_fused_backward(gp->K.ptr, gp->ld, gp->Linv.ptr, gp->n, gp->alpha.ptr, gp->flags.ptr, gp->trsv_b.ptr,
+                            gp->status.ptr, s);
     }
 }
 
-// Fit, mean and variance on the handle's streams: the overlapped pipelines
-// of the tensor-core modes, or fit then predict (FP64).  Used by the
-// host-buffer entry points and by the device-resident one alike.
+// Fit, mean and variance on the handle's streams: the overlapped pipeline of
+// the handle's mode.  Used by the host-buffer entry points and by the
+// device-resident one alike.
 void fit_predict_var(gprat_cu_gp *gp, const double *d_xt, int m, double *d_mean, double *d_var, cudaStream_t s);
 
 void loss_after_fit(gprat_cu_gp *gp, cudaStream_t s)
@@ -253,44 +194,6 @@ void loss_after_fit(gprat_cu_gp *gp, cudaStream_t s)
     else
     {
         loss_kernel(gp->y.ptr, gp->alpha.ptr, gp->K.ptr, gp->ld, gp->n, gp->params.ptr, s);
-    }
-}
-
-// Right-looking blocked solve W L^T = W (in place) over the first `rows`
-// rows of W (m x ld); if rowsq != nullptr accumulates sum_j W_ij^2.
-// row_limit(k) bounds the rows touched at block step k (triangular RHS).
-template <typename RowLimit>
-void solve_right_lt(gprat_cu_gp *gp, double *W, int64_t ldw, int rows, double *rowsq, RowLimit row_limit,
-                    cudaStream_t s)
-{
-    // Two-level blocking like the factorisation: inner 128-column steps
-    // inside a 512-column outer panel, then one K = 512 update of the rest.
-    const int n = gp->n;
-    const int64_t ld = gp->ld;
-    for (int K0 = 0; K0 < n; K0 += NBO)
-    {
-        const int bo = std::min(NBO, n - K0);
-        const int pend = K0 + bo;
-        for (int c0 = K0; c0 < pend; c0 += NB)
-        {
-            const int bs = std::min(NB, pend - c0);
-            const int k = c0 / NB;
-            const int mrows = std::min(rows, row_limit(k));
-            gemm_nt(mrows, bs, bs, W + c0, ldw, linv_block(gp, k), NB, W + c0, ldw, 1.0, 0.0, false, rowsq, s);
-            const int ncols = pend - (c0 + bs);
-            if (ncols > 0)
-            {
-                gemm_nt(mrows, ncols, bs, W + c0, ldw, kblock(gp, c0 + bs, c0), ld, W + c0 + bs, ldw, -1.0, 1.0,
-                        false, nullptr, s);
-            }
-        }
-        const int rest = n - pend;
-        if (rest > 0)
-        {
-            const int mrows = std::min(rows, row_limit((pend - 1) / NB));
-            gemm_nt(mrows, rest, bo, W + K0, ldw, kblock(gp, pend, K0), ld, W + pend, ldw, -1.0, 1.0, false, nullptr,
-                    s);
-        }
     }
 }
 
@@ -336,19 +239,19 @@ void predict_device(gprat_cu_gp *gp, const double *d_xt, int m, double *d_mean, 
     {
         StepScope step("forward KcK", s);
         GPRAT_CUDA_CHECK(cudaMemsetAsync(gp->vacc.ptr, 0, m * sizeof(double), s));
-        solve_right_lt(gp, gp->W.ptr, gp->ld, m, gp->vacc.ptr, [m](int) { return m; }, s);
+        solve_rows_fp64(gp, SolveRows{ gp->W.ptr, gp->ld, m, false, gp->vacc.ptr, nullptr, false }, s);
     }
     StepScope step("prediction uncertainty", s);
     finalize_variance(gp->vacc.ptr, m, gp->params.ptr, d_var, s);
 }
 
 // What a captured pipeline bakes in: buffer addresses (through the
-// allocation count), sizes, the mode and the schedule's knobs (every
+// allocation count), sizes, the mode, the wait budget and the schedule's knobs (every
 // GPRAT_CU_* environment variable).
 std::string pipeline_key(const gprat_cu_gp *gp, const double *d_xt, int m, const double *d_mean, const double *d_var)
 {
     char buf[256];
-    std::snprintf(buf, sizeof(buf), "%d|%d|%d|%d|%d|%d|%d|%p|%p|%p|%llu", gp->device, gp->n, m, gp->precision,
+    std::snprintf(buf, sizeof(buf), "%d|%d|%d|%d|%d|%d|%d|%d|%p|%p|%p|%llu", wait_polls(), gp->device, gp->n, m, gp->precision,
                   gp->oz_slices, gp->oz_factor_groups, gp->oz_variance_groups, static_cast<const void *>(d_xt),
                   static_cast<const void *>(d_mean), static_cast<const void *>(d_var),
                   static_cast<unsigned long long>(alloc_generation()));
@@ -465,10 +368,14 @@ void fit_predict_var(gprat_cu_gp *gp, const double *d_xt, int m, double *d_mean,
     {
         fit_predict_graphed(fit_predict_oz, gp, d_xt, m, d_mean, d_var, s);
     }
-    else
+    else if (steps_enabled())
     {
         fit(gp, s);
         predict_device(gp, d_xt, m, d_mean, d_var, s);
+    }
+    else
+    {
+        fit_predict_graphed(fit_predict_fp64, gp, d_xt, m, d_mean, d_var, s);
     }
 }
 
@@ -477,15 +384,16 @@ void finish_and_check(gprat_cu_gp *gp)
     GPRAT_CUDA_CHECK(
         cudaMemcpyAsync(gp->h_status, gp->status.ptr, sizeof(DeviceStatus), cudaMemcpyDeviceToHost, gp->stream));
     GPRAT_CUDA_CHECK(cudaStreamSynchronize(gp->stream));
+    // a timeout first: the values after it mean nothing
+    if (gp->h_status->timeout != 0)
+    {
+        throw Error(GPRAT_CU_ERR_TIMEOUT, "a bounded device wait timed out");
+    }
     if (gp->h_status->not_spd_row != 0)
     {
         throw Error(GPRAT_CU_ERR_NOT_SPD, "Cholesky factorisation failed: covariance matrix is not positive definite "
                                           "(non-positive pivot at row " +
                                               std::to_string(gp->h_status->not_spd_row - 1) + ")");
-    }
-    if (gp->h_status->timeout != 0)
-    {
-        throw Error(GPRAT_CU_ERR_TIMEOUT, "a bounded device wait timed out");
     }
 }
 
@@ -512,19 +420,19 @@ void download(gprat_cu_gp *gp, double *host, const double *dev, int64_t count)
 
 void gradient_device(gprat_cu_gp *gp, bool adam, cudaStream_t s)
 {
-    // the adjoint gradient and Adam always run in FP64
-    factor_fp64(gp, s);
-    solve_alpha_fp64(gp, s);
-    loss_kernel(gp->y.ptr, gp->alpha.ptr, gp->K.ptr, gp->ld, gp->n, gp->params.ptr, s);
-    // U = L^-T: solve U L^T = I; column block k of U has nonzeros in rows < (k+1)*NB
+    // the adjoint gradient and Adam always run in FP64.  U = L^-T (the solve
+    // U L^T = I) and z = L^-1 y come with the factorisation; alpha = U z.
     gp->U.ensure(static_cast<int64_t>(gp->n) * gp->ld);
     set_identity(gp->U.ptr, gp->ld, gp->n, s);
-    solve_right_lt(gp, gp->U.ptr, gp->ld, gp->n, nullptr, [](int k) { return (k + 1) * NB; }, s);
-    const int t = ceil_div(gp->n, 128);
+    factor_forward_fp64(gp, SolveRows{ gp->U.ptr, gp->ld, gp->n, true, nullptr, nullptr, false }, s);
+    cross_times_alpha(gp->U.ptr, gp->ld, gp->n, gp->n, gp->z.ptr, gp->alpha.ptr, s, true);
+    // y . alpha = z . z
+    loss_kernel(gp->z.ptr, gp->z.ptr, gp->K.ptr, gp->ld, gp->n, gp->params.ptr, s);
+    const int t = ceil_div(gp->n, 64);
     gp->partials.ensure(static_cast<int64_t>(t) * (t + 1) / 2 * 3);
     int np = 0;
     adjoint_trace(gp->U.ptr, gp->ld, gp->alpha.ptr, gp->x.ptr, gp->n, gp->d, gp->params.ptr, gp->partials.ptr, &np,
-                  s);
+                  gp->status.ptr, s);
     adjoint_finish(gp->partials.ptr, np, gp->n, gp->params.ptr, adam, s);
 }
 
@@ -662,13 +570,13 @@ void gp_check(gprat_cu_gp *gp, cudaStream_t s)
 {
     GPRAT_CUDA_CHECK(cudaMemcpyAsync(gp->h_status, gp->status.ptr, sizeof(DeviceStatus), cudaMemcpyDeviceToHost, s));
     GPRAT_CUDA_CHECK(cudaStreamSynchronize(s));
-    if (gp->h_status->not_spd_row != 0)
-    {
-        throw Error(GPRAT_CU_ERR_NOT_SPD, "Cholesky factorisation failed: covariance matrix is not positive definite");
-    }
     if (gp->h_status->timeout != 0)
     {
         throw Error(GPRAT_CU_ERR_TIMEOUT, "a bounded device wait timed out");
+    }
+    if (gp->h_status->not_spd_row != 0)
+    {
+        throw Error(GPRAT_CU_ERR_NOT_SPD, "Cholesky factorisation failed: covariance matrix is not positive definite");
     }
 }
 
@@ -985,7 +893,16 @@ int gprat_cu_cholesky(gprat_cu_gp *gp, const double hyper[3], double *tiles_out)
             DeviceGuard guard(gp->device);
             StepPrefix prefix("cholesky_step");
             upload_hyper(gp, hyper, gp->stream);
-            factor_fp64(gp, gp->stream);
+            // The factor itself is the result, compared entry by entry with the
+            // reference's.  Subtracting the products one by one keeps the error of
+            // an entry that cancels to next to nothing in step with what is left of
+            // it: the smallest entries (1e-7 at n = 32768) agree with the
+            // reference's to 3e-11, against 5e-10 with sums subtracted, although
+            // those are closer over all entries (root mean square 7e-17 against
+            // 5e-16).
+            SolveRows none{};
+            none.c_first = true;
+            factor_fp64(gp, none, gp->stream);
             std::vector<double> full(static_cast<size_t>(gp->n) * gp->ld);
             download(gp, full.data(), gp->K.ptr, static_cast<int64_t>(gp->n) * gp->ld);
             finish_and_check(gp);
@@ -1104,21 +1021,14 @@ int gprat_cu_predict_full_covariance(gprat_cu_gp *gp, const double hyper[3], con
             DevBuf<double> S;
             S.ensure(static_cast<int64_t>(m) * lds);
             assemble_prior(gp->xt.ptr, m, gp->d, gp->params.ptr, S.ptr, lds, gp->stream);
-            GemmArgs a{};
-            a.M = m;
-            a.N = m;
-            a.K = gp->n;
-            a.A = gp->W.ptr;
-            a.lda = gp->ld;
-            a.transA = false;
+            UpdateArgs a{};
+            a.rows[0] = RowGroup{ gp->W.ptr, gp->ld, S.ptr, lds, m };
             a.B = gp->W.ptr;
             a.ldb = gp->ld;
-            a.transB = true;
-            a.C = S.ptr;
-            a.ldc = lds;
-            a.alpha = -1.0;
-            a.beta = 1.0;
-            dgemm(a, gp->stream);
+            a.N = m;
+            a.K = gp->n;
+            a.status = gp->status.ptr;
+            dgemm_update(a, gp->stream);
             download(gp, mean, gp->mean.ptr, m);
             GPRAT_CUDA_CHECK(cudaMemcpy2DAsync(cov, m * sizeof(double), S.ptr, lds * sizeof(double),
                                                m * sizeof(double), m, cudaMemcpyDeviceToHost, gp->stream));
@@ -1136,8 +1046,17 @@ int gprat_cu_compute_loss(gprat_cu_gp *gp, const double hyper[3], double *loss)
             require(loss != nullptr, "loss must not be NULL");
             DeviceGuard guard(gp->device);
             upload_hyper(gp, hyper, gp->stream);
-            fit(gp, gp->stream);
-            loss_after_fit(gp, gp->stream);
+            if (gp->precision == GPRAT_CU_PREC_FP64 && !steps_enabled())
+            {
+                // y . alpha = z . z: no backward solve
+                factor_forward_fp64(gp, SolveRows{}, gp->stream);
+                loss_kernel(gp->z.ptr, gp->z.ptr, gp->K.ptr, gp->ld, gp->n, gp->params.ptr, gp->stream);
+            }
+            else
+            {
+                fit(gp, gp->stream);
+                loss_after_fit(gp, gp->stream);
+            }
             GPRAT_CUDA_CHECK(cudaMemcpyAsync(gp->h_params, gp->params.ptr, sizeof(DeviceParams),
                                              cudaMemcpyDeviceToHost, gp->stream));
             finish_and_check(gp);

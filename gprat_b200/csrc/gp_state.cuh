@@ -17,7 +17,7 @@ namespace gprat_cu
 {
 
 constexpr int NB = 128;   // diagonal block size (potrf + inverse)
-constexpr int NBO = 512;  // outer block of the two-level factorisation and solves
+constexpr int NBO = 512;  // outer block of the two-level solves
 
 // Device memory of the library's buffers.  Allocation is stream-ordered on a
 // private stream of the current device (cudaMallocAsync from the device's
@@ -101,7 +101,7 @@ struct gprat_cu_gp
 
     // FP64 path
     gprat_cu::DevBuf<double> x, y, K, Linv, alpha, U, partials;
-    gprat_cu::DevBuf<double> xt, W, vacc, mean_part, mean, var, losses;
+    gprat_cu::DevBuf<double> xt, W, vacc, mean_part, mean, var, losses, z;
     gprat_cu::DevBuf<gprat_cu::DeviceParams> params;
     gprat_cu::DevBuf<gprat_cu::DeviceStatus> status;
     gprat_cu::DeviceParams *h_params = nullptr;
@@ -153,7 +153,7 @@ struct gprat_cu_gp
             cudaStreamSynchronize(vstream);
         }
         for (gprat_cu::DevBuf<double> *b : { &x, &y, &K, &Linv, &alpha, &U, &partials, &xt, &W, &vacc, &mean_part,
-                                             &mean, &var, &losses, &D64, &pcg_r, &pcg_z, &pcg_p, &pcg_q, &symv_part, &trsv_b })
+                                             &mean, &var, &losses, &z, &D64, &pcg_r, &pcg_z, &pcg_p, &pcg_q, &symv_part, &trsv_b })
         {
             b->release();
         }
@@ -255,6 +255,27 @@ int sm_percent(const char *name, int dflt);
 void ensure_lookahead(gprat_cu_gp *gp, int nevents);
 // Events one look-ahead pipeline over n training points uses.
 int lookahead_events(int n);
+
+// fp64_path.cu: the FP64 factorisation and solves.
+// Rows solved against the factor, E L^T = E in place.
+struct SolveRows
+{
+    double *ptr;     // rows x n, ld
+    int64_t ld;
+    int rows;
+    bool identity;   // E starts as the identity: row i is zero left of column i
+    double *rowsq;   // optional: += sum_j E_ij^2 of the solution
+    double *vec;     // optional: n values, vec := L^-1 vec
+    bool c_first;    // see UpdateArgs
+};
+// Factors the covariance in K (in place, with Linv) and solves e's rows and
+// vector in the same launches.  rows_ready (optional): recorded once e's rows
+// and vector are ready.
+void factor_solve_fp64(gprat_cu_gp *gp, const SolveRows &e, cudaStream_t s, cudaEvent_t rows_ready = nullptr);
+// The solve alone, with the factor in K.
+void solve_rows_fp64(gprat_cu_gp *gp, const SolveRows &e, cudaStream_t s);
+// Fit, mean and variance.
+void fit_predict_fp64(gprat_cu_gp *gp, const double *d_xt, int m, double *d_mean, double *d_var, cudaStream_t s);
 
 // ozaki_path.cu: the FP64-accurate pipeline on the int8 tensor cores
 // (GPRAT_CU_PREC_FP64_INT8).  The factor is FP64 (in K, with Linv), every

@@ -172,35 +172,23 @@ extern "C" int gprat_cu_compute_loss_noalloc(int device,
             {
                 continue;
             }
-            GemmArgs pa{};
-            pa.M = rows;
-            pa.N = bs;
-            pa.K = bs;
-            pa.A = K + (r0 + bs) * ld + r0;
-            pa.lda = ld;
-            pa.B = Lk;
-            pa.ldb = NB;
-            pa.transB = true;
-            pa.C = K + (r0 + bs) * ld + r0;
-            pa.ldc = ld;
-            pa.alpha = 1.0;
-            pa.beta = 0.0;
-            dgemm(pa, s);
-            GemmArgs ta{};
-            ta.M = rows;
+            double *panel = K + (r0 + bs) * ld + r0;
+            SolveArgs pa{};
+            pa.rows[0] = RowGroup{ panel, ld, panel, ld, rows };
+            pa.Linv = Lk;
+            pa.ldi = NB;
+            pa.bs = bs;
+            pa.status = status;
+            dgemm_solve(pa, s);
+            UpdateArgs ta{};
+            ta.rows[0] = RowGroup{ panel, ld, panel + bs, ld, rows };
+            ta.B = panel;
+            ta.ldb = ld;
             ta.N = rows;
             ta.K = bs;
-            ta.A = K + (r0 + bs) * ld + r0;
-            ta.lda = ld;
-            ta.B = K + (r0 + bs) * ld + r0;
-            ta.ldb = ld;
-            ta.transB = true;
-            ta.C = K + (r0 + bs) * ld + r0 + bs;
-            ta.ldc = ld;
-            ta.alpha = -1.0;
-            ta.beta = 1.0;
             ta.lower = true;
-            dgemm(ta, s);
+            ta.status = status;
+            dgemm_update(ta, s);
         }
         GPRAT_CUDA_CHECK(cudaMemcpyAsync(alpha, d_train_out, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
         trsv_forward(K, ld, Linv, NB, n, alpha, nullptr, s);
@@ -210,6 +198,10 @@ extern "C" int gprat_cu_compute_loss_noalloc(int device,
         DeviceStatus st{};
         GPRAT_CUDA_CHECK(cudaMemcpyAsync(&st, status, sizeof(DeviceStatus), cudaMemcpyDeviceToHost, s));
         GPRAT_CUDA_CHECK(cudaStreamSynchronize(s));
+        if (st.timeout != 0)
+        {
+            throw Error(GPRAT_CU_ERR_TIMEOUT, "a bounded device wait timed out");
+        }
         if (st.not_spd_row != 0)
         {
             throw Error(GPRAT_CU_ERR_NOT_SPD, "Cholesky factorisation failed: covariance matrix is not positive "

@@ -1,13 +1,14 @@
 // Kernel-level test entry points of the C ABI (gprat_cu_test_*): run one
 // kernel on host-provided data so that tests can compare it in isolation
-// (tcgen05 TF32/BF16 GEMM, fused triangular solves, the int8 digit split and
-// the int8-emulated FP64 GEMM).
+// (tcgen05 TF32/BF16 GEMM, the FP64 update and panel solve, fused triangular
+// solves, the int8 digit split and the int8-emulated FP64 GEMM).
 #include "common.cuh"
 #include "gprat_cu.h"
 #include "ozaki.cuh"
 #include "tc_gemm.cuh"
 
 #include <algorithm>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -392,7 +393,7 @@ extern "C" int gprat_cu_test_set_wait_budget(int64_t polls)
 {
     try
     {
-        set_trsv_wait_budget(polls);
+        set_wait_budget(polls);
         set_last_error("");
         return GPRAT_CU_OK;
     }
@@ -400,5 +401,157 @@ extern "C" int gprat_cu_test_set_wait_budget(int64_t polls)
     {
         set_last_error(e.what());
         return e.code;
+    }
+}
+
+extern "C" int gprat_cu_test_dgemm_update(int m0, int m1, int N, int K, const double *A0, const double *A1,
+                                          const double *B, double *C0, double *C1, int lower, const double *z,
+                                          double *y, int tile)
+{
+    try
+    {
+        if (m0 < 0 || m1 < 0 || m0 + m1 <= 0 || N <= 0 || K <= 0 || (m0 > 0 && (A0 == nullptr || C0 == nullptr)) ||
+            (m1 > 0 && (A1 == nullptr || C1 == nullptr)) || B == nullptr || (lower != 0 && m0 < N) ||
+            (z == nullptr) != (y == nullptr) || tile < 0 || tile > 2)
+        {
+            throw Error(GPRAT_CU_ERR_INVALID_ARG, "gprat_cu_test_dgemm_update: invalid arguments");
+        }
+        cudaStream_t s = nullptr;
+        const int64_t lk = round_up(K, 8), ln = round_up(N, 8);
+        // the padding columns hold NaN: nothing may read them as data
+        auto upload = [&](int rows, int cols, int64_t ld, const double *src)
+        {
+            auto b = std::make_unique<Buf>(std::max<size_t>(static_cast<size_t>(rows) * ld * 8, 16));
+            GPRAT_CUDA_CHECK(cudaMemset(b->p, 0xff, static_cast<size_t>(rows) * ld * 8));
+            if (rows > 0)
+            {
+                GPRAT_CUDA_CHECK(cudaMemcpy2D(b->p, ld * 8, src, cols * 8, cols * 8, rows, cudaMemcpyHostToDevice));
+            }
+            return b;
+        };
+        auto dA0 = upload(m0, K, lk, A0), dA1 = upload(m1, K, lk, A1), dB = upload(N, K, lk, B);
+        auto dC0 = upload(m0, N, ln, C0), dC1 = upload(m1, N, ln, C1);
+        auto dz = upload(z != nullptr ? 1 : 0, K, K, z), dy = upload(y != nullptr ? 1 : 0, N, N, y);
+        Buf dStatus(sizeof(DeviceStatus));
+        GPRAT_CUDA_CHECK(cudaMemset(dStatus.p, 0, sizeof(DeviceStatus)));
+        UpdateArgs a{};
+        a.rows[0] = RowGroup{ static_cast<double *>(dA0->p), lk, static_cast<double *>(dC0->p), ln, m0 };
+        a.rows[1] = RowGroup{ static_cast<double *>(dA1->p), lk, static_cast<double *>(dC1->p), ln, m1 };
+        a.B = static_cast<double *>(dB->p);
+        a.ldb = lk;
+        a.N = N;
+        a.K = K;
+        a.lower = lower != 0;
+        a.z = z != nullptr ? static_cast<double *>(dz->p) : nullptr;
+        a.y = y != nullptr ? static_cast<double *>(dy->p) : nullptr;
+        a.status = static_cast<DeviceStatus *>(dStatus.p);
+        a.tile = tile;
+        dgemm_update(a, s);
+        GPRAT_CUDA_CHECK(cudaStreamSynchronize(s));
+        DeviceStatus st{};
+        GPRAT_CUDA_CHECK(cudaMemcpy(&st, dStatus.p, sizeof(st), cudaMemcpyDeviceToHost));
+        if (st.timeout != 0)
+        {
+            throw Error(GPRAT_CU_ERR_TIMEOUT, "FP64 update: a bounded wait timed out");
+        }
+        if (m0 > 0)
+        {
+            GPRAT_CUDA_CHECK(cudaMemcpy2D(C0, N * 8, dC0->p, ln * 8, N * 8, m0, cudaMemcpyDeviceToHost));
+        }
+        if (m1 > 0)
+        {
+            GPRAT_CUDA_CHECK(cudaMemcpy2D(C1, N * 8, dC1->p, ln * 8, N * 8, m1, cudaMemcpyDeviceToHost));
+        }
+        if (y != nullptr)
+        {
+            GPRAT_CUDA_CHECK(cudaMemcpy(y, dy->p, N * 8, cudaMemcpyDeviceToHost));
+        }
+        set_last_error("");
+        return GPRAT_CU_OK;
+    }
+    catch (const Error &e)
+    {
+        set_last_error(e.what());
+        return e.code;
+    }
+    catch (const std::exception &e)
+    {
+        set_last_error(e.what());
+        return GPRAT_CU_ERR_INVALID_ARG;
+    }
+}
+
+extern "C" int gprat_cu_test_dgemm_solve(int m0, int m1, int bs, double *P0, double *P1, const double *Linv,
+                                         double *rowsq, double *y, int tile)
+{
+    try
+    {
+        if (m0 < 0 || m1 < 0 || (m0 + m1 <= 0 && y == nullptr) || bs <= 0 || bs > 128 || (m0 > 0 && P0 == nullptr) ||
+            (m1 > 0 && P1 == nullptr) || Linv == nullptr || (tile != 0 && tile != 1 && tile != 2 && tile != 4))
+        {
+            throw Error(GPRAT_CU_ERR_INVALID_ARG, "gprat_cu_test_dgemm_solve: invalid arguments");
+        }
+        cudaStream_t s = nullptr;
+        const int64_t ld = 128;
+        auto upload = [&](int rows, int cols, int64_t l, const double *src)
+        {
+            auto b = std::make_unique<Buf>(std::max<size_t>(static_cast<size_t>(rows) * l * 8, 16));
+            GPRAT_CUDA_CHECK(cudaMemset(b->p, 0xff, static_cast<size_t>(rows) * l * 8));
+            if (rows > 0)
+            {
+                GPRAT_CUDA_CHECK(cudaMemcpy2D(b->p, l * 8, src, cols * 8, cols * 8, rows, cudaMemcpyHostToDevice));
+            }
+            return b;
+        };
+        auto d0 = upload(m0, bs, ld, P0), d1 = upload(m1, bs, ld, P1), dL = upload(bs, bs, ld, Linv);
+        auto dr = upload(rowsq != nullptr && m1 > 0 ? 1 : 0, m1, m1, rowsq), dy = upload(y != nullptr ? 1 : 0, bs, bs, y);
+        Buf dStatus(sizeof(DeviceStatus));
+        GPRAT_CUDA_CHECK(cudaMemset(dStatus.p, 0, sizeof(DeviceStatus)));
+        SolveArgs a{};
+        a.rows[0] = RowGroup{ static_cast<double *>(d0->p), ld, static_cast<double *>(d0->p), ld, m0 };
+        a.rows[1] = RowGroup{ static_cast<double *>(d1->p), ld, static_cast<double *>(d1->p), ld, m1 };
+        a.Linv = static_cast<double *>(dL->p);
+        a.ldi = ld;
+        a.bs = bs;
+        a.rowsq = rowsq != nullptr ? static_cast<double *>(dr->p) : nullptr;
+        a.y = y != nullptr ? static_cast<double *>(dy->p) : nullptr;
+        a.status = static_cast<DeviceStatus *>(dStatus.p);
+        a.tile = tile;
+        dgemm_solve(a, s);
+        GPRAT_CUDA_CHECK(cudaStreamSynchronize(s));
+        DeviceStatus st{};
+        GPRAT_CUDA_CHECK(cudaMemcpy(&st, dStatus.p, sizeof(st), cudaMemcpyDeviceToHost));
+        if (st.timeout != 0)
+        {
+            throw Error(GPRAT_CU_ERR_TIMEOUT, "FP64 panel solve: a bounded wait timed out");
+        }
+        if (m0 > 0)
+        {
+            GPRAT_CUDA_CHECK(cudaMemcpy2D(P0, bs * 8, d0->p, ld * 8, bs * 8, m0, cudaMemcpyDeviceToHost));
+        }
+        if (m1 > 0)
+        {
+            GPRAT_CUDA_CHECK(cudaMemcpy2D(P1, bs * 8, d1->p, ld * 8, bs * 8, m1, cudaMemcpyDeviceToHost));
+        }
+        if (rowsq != nullptr && m1 > 0)
+        {
+            GPRAT_CUDA_CHECK(cudaMemcpy(rowsq, dr->p, m1 * 8, cudaMemcpyDeviceToHost));
+        }
+        if (y != nullptr)
+        {
+            GPRAT_CUDA_CHECK(cudaMemcpy(y, dy->p, bs * 8, cudaMemcpyDeviceToHost));
+        }
+        set_last_error("");
+        return GPRAT_CU_OK;
+    }
+    catch (const Error &e)
+    {
+        set_last_error(e.what());
+        return e.code;
+    }
+    catch (const std::exception &e)
+    {
+        set_last_error(e.what());
+        return GPRAT_CU_ERR_INVALID_ARG;
     }
 }

@@ -26,6 +26,9 @@
 // sets the status word's timeout flag (the caller reports an error).
 #include "common.cuh"
 
+#include <algorithm>
+#include <atomic>
+
 namespace gprat_cu
 {
 namespace
@@ -969,10 +972,29 @@ void trsv_fused_backward_f32(const float *L, int64_t ld, const float *Linv, int 
 // Sets the poll budget of the solves' waits on the current device; polls < 0
 // restores the default.  Test use: a budget of 0 makes a wait on an unsolved
 // block give up at once (the status word's timeout flag), with no hang.
-void set_trsv_wait_budget(long long polls)
+namespace
 {
+constexpr int MAX_DEVICES = 64;
+std::atomic<int> g_wait_polls[MAX_DEVICES];  // budget + 1; 0: the default
+}  // namespace
+
+void set_wait_budget(long long polls)
+{
+    int dev = 0;
+    GPRAT_CUDA_CHECK(cudaGetDevice(&dev));
+    if (dev < MAX_DEVICES)
+    {
+        g_wait_polls[dev].store(polls < 0 ? 0 : static_cast<int>(std::min(polls, 1ll << 30)) + 1);
+    }
     const long long v = polls < 0 ? SPIN_LIMIT : polls;
     GPRAT_CUDA_CHECK(cudaMemcpyToSymbol(g_spin_limit, &v, sizeof(v)));
+}
+
+int wait_polls()
+{
+    int dev = 0;
+    GPRAT_CUDA_CHECK(cudaGetDevice(&dev));
+    return dev < MAX_DEVICES ? g_wait_polls[dev].load(std::memory_order_relaxed) - 1 : -1;
 }
 
 }  // namespace gprat_cu

@@ -318,6 +318,40 @@ int gprat_cu_test_tc_gemm(int kind,
                           int tile_mode);
 
 /*
+ * Kernel-level test entries (no counterpart in the reference): the FP64
+ * update and panel solve of the factorisation on the current device, with
+ * dense row-major host matrices.  update: C0 -= A0 B^T (m0 x N; lower != 0:
+ * only C0[i][j], j <= i, m0 >= N) and C1 -= A1 B^T (m1 x N), with B N x K; y
+ * (optional, with z): y -= B z.  tile: 0 = the library's choice, 1 = 64 x 64,
+ * 2 = 32 x 32.  solve: P0 (m0 x bs) and P1 (m1 x bs) := P Linv^T with the lower
+ * triangular Linv (bs x bs, bs <= 128); rowsq (optional): rowsq[i] +=
+ * sum_j P1_new[i][j]^2; y (optional): y := Linv y.  tile: 0 = the library's
+ * choice, 1, 2, 4 = 16, 32, 64 rows per CTA.
+ */
+int gprat_cu_test_dgemm_update(int m0,
+                               int m1,
+                               int N,
+                               int K,
+                               const double *A0,
+                               const double *A1,
+                               const double *B,
+                               double *C0,
+                               double *C1,
+                               int lower,
+                               const double *z,
+                               double *y,
+                               int tile);
+int gprat_cu_test_dgemm_solve(int m0,
+                              int m1,
+                              int bs,
+                              double *P0,
+                              double *P1,
+                              const double *Linv,
+                              double *rowsq,
+                              double *y,
+                              int tile);
+
+/*
  * Kernel-level test entry (no counterpart in the reference): the
  * single-launch blocked triangular solves of the library on the current
  * device.  L: n x n row-major host matrix whose lower triangle (diagonal
@@ -331,11 +365,13 @@ int gprat_cu_test_trsv(int kind, int n, const double *L, const double *b, double
 
 /*
  * Test entry (no counterpart in the reference, which bounds no wait): the
- * number of polls after which a wait of the single-launch triangular solves
- * on an unsolved row block gives up, on the current device; the call then
- * returns GPRAT_CU_ERR_TIMEOUT.  polls < 0 restores the default (about
- * 0.5-1 s of polling).  The waits only re-read global memory, so a budget of
- * 0 ends them at once and nothing is left in flight.
+ * number of polls after which a wait gives up on the current device: of the
+ * single-launch triangular solves on an unsolved row block, and of the FP64
+ * products on the copies of their operands; the call then returns
+ * GPRAT_CU_ERR_TIMEOUT.  polls < 0 restores the defaults (about 0.5-1 s and
+ * 2 s).  A product's CTA whose wait gave up issues no further copy and stays
+ * until those in flight have landed, so a budget of 0 leaves nothing in
+ * flight.
  */
 int gprat_cu_test_set_wait_budget(int64_t polls);
 
