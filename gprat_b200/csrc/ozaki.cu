@@ -22,26 +22,40 @@
 //     resident until its last group, so every digit tile crosses from L2
 //     once per block; the spare slots let the next block's first planes load
 //     while the current block's last groups run.
-//   warps 1 and 2, one lane each (leader): MMA issuers, taking alternate
-//     groups so that one thread's barrier waits do not idle the tensor core
-//     (the issuer below says why).  Group g of block k is one unit:
-//     for p = 0..g, four tcgen05.mma.cta_group::2.kind::i8 (M 256, N 128,
-//     K 32) of A_p against B_{g-p} into one int32 accumulator in tensor
-//     memory (four accumulators of 128 columns rotate); tcgen05.commit frees
-//     the accumulator, and after the block (from both issuers) its slots.
+//   warp 2 (leader): scout.  Waits for what each unit needs and signals the
+//     issuer through a hardware barrier, so that the thread that runs in step
+//     with the tensor core tests no shared-memory barrier.
+//   warp 1, one lane (leader): MMA issuer.  Group g of block k is one unit,
+//     taken from the highest group down: for p = 0..g, four
+//     tcgen05.mma.cta_group::2.kind::i8 (M 256, N 128, K 32) of A_p against
+//     B_{g-p} into one int32 accumulator in tensor memory (four accumulators
+//     of 128 columns rotate), all 2 G (G + 1) of a block unrolled;
+//     tcgen05.commit frees plane g's slot and tells the epilogue.
 //   warps 4..11 (both CTAs): epilogue.  Two warps per TMEM lane quarter, 64
-//     columns each (224 registers after setmaxnreg); units are read with
-//     double-buffered tcgen05.ld, 16 columns at a time, in pairs of groups
-//     (g, g + 1) and combined exactly in int32 as 254 P_g + P_{g+1} (at
-//     most 2,112,012,032), converted exactly to FP64 (2^52 + 2^31 bias
-//     trick) and added by one FMA with the pair's scale
-//     2^(eA + eB - 12) / 254^(g + 1) into 64 FP64 registers per thread (a
-//     last unpaired group as 254 P_g at the same scale).  The next block's
-//     exponents are loaded while a block is read.  After the tile's last
-//     unit, alpha * acc is written from the registers, 8 columns at a time,
-//     each lane its own row with 16-byte stores (beta = 1 adds to C; those C
+//     columns each (224 registers after setmaxnreg).  3 and 5 groups: the two
+//     highest are combined exactly in int32 as 254 P_{G-2} + P_{G-1}, kept in
+//     registers while the others are multiplied, and the block's whole sum is
+//     formed exactly in 64-bit integers, turned into FP64 by one subtraction
+//     and added by one FMA with the scale 2^(eA + eB - 12) / 254^(G - 1) into
+//     64 FP64 accumulators per thread.  Other G: pairs of groups, each
+//     converted and added so (at most 2,112,012,032 in int32).  The next
+//     block's exponents are loaded while a block is read.  After the tile's
+//     last unit, alpha * acc is written from the registers, 8 columns at a
+//     time, each lane its own row with 16-byte stores (beta = 1 adds to C,
+//     whose lines were sent for when the tile began; those C
 //     values are loaded first); the shared memory a staging transpose would
 //     take holds a ninth digit-plane slot instead.
+// What bounds it: the epilogue.  FP64 instructions take 3.2 times as long
+// while int8 MMAs stream (12 cycles a warp instruction and scheduler instead
+// of 4), and so do integer ones between them, so what counts is the FP64
+// instructions per element and block: 2 here (5 groups), 6 when each pair of
+// groups is converted by itself.  One 256 x 128 x 128 block of 5 groups takes
+// 8400 cycles, of which its MMAs are 3840 (64 each); with the epilogue's
+// arithmetic left out 5400, with the integer sums alone 7100.  At 8192^3, 5
+// groups, 1785 -> 2032 TOP/s against two issuing threads that waited for the
+// barriers themselves and three pairs per block; lower 28672^2 x 2048: 1603 ->
+// 1783; 8192 x 128 x 1920: 96.2 -> 87 us; 3 groups 1293 -> 1405.  4 groups: 1650 to
+// 1800 from run to run (before 1720).
 // Every mbarrier wait is bounded (tcgen05_ptx.cuh); a wait that gives up
 // raises the CTA's abort flag, the roles leave their loops, TMA copies in
 // flight get 200 us to land, the MMA issuer drains, TMEM is freed and the
@@ -243,6 +257,7 @@ constexpr int OZ_A_BYTES = 128 * 128;  // 128 rows x 128 digit bytes
 constexpr int OZ_B_BYTES = 64 * 128;   // this CTA's half of the 128 B rows
 constexpr int OZ_RING = 9;  // slots of one A and one B digit plane (>= s + 1: the next block's first planes load early)
 constexpr int OZ_NACC = 4;             // int32 accumulators of 128 TMEM columns
+constexpr int OZ_NPHASE = 4;           // barriers of the epilogue's phases, in turn
 constexpr int OZ_TMEM_COLS = OZ_NACC * 128;
 constexpr int OZ_SMEM_BYTES =
     1024 + OZ_RING * (OZ_A_BYTES + OZ_B_BYTES) + 512;
@@ -252,6 +267,37 @@ static_assert(OZ_RING >= OZ_MAX_SLICES + 1, "the ring must hold one block's plan
 constexpr uint32_t OZ_IDESC =
     (2u << 4) | (1u << 7) | (1u << 10) | ((128u >> 3) << 17) | ((256u >> 4) << 24);
 constexpr int OZ_GROUP_M = 8;  // row tiles per group of the non-lower tile order
+
+// Whether the epilogue sums a block's groups in 64-bit integers: where that
+// saves FP64 instructions enough to pay for its two widening multiplications.
+// 3 groups: 1405 TOP/s at 8192^3 against 1300 in pairs; 5: 2030 against 1800;
+// 4: 1615 against 1700, so pairs; above 5 the sum has more than 52 bits.
+constexpr bool oz_sums(int G)
+{
+    return G == 3 || G == 5;
+}
+
+// Whether unit j of a block's G (groups G - 1 .. 0) ends a phase, after which
+// the epilogue reads it and the units since the phase before.  With the sums
+// the phases are the two highest groups and the rest; else pairs from the top,
+// whose sum 254 P_{g-1} + P_g is exact in int32 up to the pair (5, 4), so
+// group 6 is alone.
+__host__ __device__ constexpr bool phase_ends(int j, int G)
+{
+    return j == G - 1 || (oz_sums(G) ? j == 1 : ((j & 1) != 0) == (G != 7));
+}
+
+// The scout's signal to the MMA issuer: a hardware barrier of their two warps
+// per accumulator.
+constexpr int OZ_SCOUT_BAR = 1;
+__device__ __forceinline__ void scout_arrive(int u)
+{
+    asm volatile("bar.arrive %0, 64;" ::"r"(OZ_SCOUT_BAR + u) : "memory");
+}
+__device__ __forceinline__ void scout_sync(int u)
+{
+    asm volatile("bar.sync %0, 64;" ::"r"(OZ_SCOUT_BAR + u) : "memory");
+}
 
 struct OzKernelArgs
 {
@@ -308,13 +354,27 @@ __device__ __forceinline__ void tmem_ld16_i(uint32_t taddr, int32_t *v)
     }
 }
 
+__device__ __forceinline__ void tmem_ld8_i(uint32_t taddr, int32_t (&v)[8])
+{
+    uint32_t r[8];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr));
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+    {
+        v[j] = static_cast<int32_t>(r[j]);
+    }
+}
+
 // Ties registers written by tcgen05.ld to the point after tcgen05.wait::ld:
 // an empty volatile asm that reads and writes each one, so that no use is
 // scheduled before the wait.
-__device__ __forceinline__ void regs_loaded(int32_t (&v)[16])
+template <int N>
+__device__ __forceinline__ void regs_loaded(int32_t (&v)[N])
 {
 #pragma unroll
-    for (int j = 0; j < 16; ++j)
+    for (int j = 0; j < N; ++j)
     {
         asm volatile("" : "+r"(v[j]));
     }
@@ -324,6 +384,28 @@ __device__ __forceinline__ void regs_loaded(int32_t (&v)[16])
 __device__ __forceinline__ double i2d(int32_t v)
 {
     return __dsub_rn(__hiloint2double(0x43300000, v ^ static_cast<int32_t>(0x80000000u)), I2D_BIAS);
+}
+
+// The sum of a block's G groups, V = sum_g 254^(G-1-g) P_g with |V| < 2^51
+// (at most 2.217e15 of 2.252e15), as FP64: low = 254 P_{G-2} + P_{G-1} and the
+// groups above it added in 64-bit integers to the bit pattern of
+// 1.5 * 2^52 (+ 2^31, so that low enters as an unsigned word), which is then
+// the pattern of 1.5 * 2^52 + 2^31 + V.
+constexpr double V2D_BIAS = 6755399441055744.0 + 2147483648.0;
+template <int G>
+__device__ __forceinline__ double sum_of_groups(int32_t p0, int32_t p1, int32_t p2, int32_t low)
+{
+    int64_t v = (static_cast<int64_t>(0x43380000) << 32) | static_cast<uint32_t>(low ^ static_cast<int32_t>(0x80000000u));
+    if (G == 3)
+    {
+        v += static_cast<int64_t>(p0) * (OZ_IBASE * OZ_IBASE);
+    }
+    else
+    {
+        v += static_cast<int64_t>(p2) * (OZ_IBASE * OZ_IBASE);
+        v += static_cast<int64_t>(p0 * OZ_IBASE + p1) * (OZ_IBASE * OZ_IBASE * OZ_IBASE);
+    }
+    return __dsub_rn(__longlong_as_double(v), V2D_BIAS);
 }
 
 // pair tile t -> (m0, n0): 256-row x 128-column tiles.  Lower mode: row tile i
@@ -355,6 +437,8 @@ __device__ __forceinline__ void oz_tile(int t, bool lower, int tiles_m, int tile
     n0 = (t - i * (i + 1)) * 128;
 }
 
+// G: the number of groups.
+template <int G>
 __global__ void __launch_bounds__(OZ_THREADS, 1)
     oz_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, OzKernelArgs p)
 {
@@ -364,8 +448,8 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     uint8_t *bring = aring + OZ_RING * OZ_A_BYTES;
     uint64_t *full = reinterpret_cast<uint64_t *>(bring + OZ_RING * OZ_B_BYTES);
     uint64_t *empty = full + OZ_RING;
-    uint64_t *tfull = empty + OZ_RING;
-    uint64_t *tempty = tfull + OZ_NACC;
+    uint64_t *pfull = empty + OZ_RING;
+    uint64_t *tempty = pfull + OZ_NPHASE;
     uint64_t *drain = tempty + OZ_NACC;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(drain + 1);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
@@ -376,21 +460,24 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     const bool leader = rank == 0;
     const int pair = blockIdx.x >> 1;
     const int npairs = gridDim.x >> 1;
-    const int G = p.groups;
+    constexpr bool SUM = oz_sums(G);
 
     if (threadIdx.x == 0)
     {
         for (int i = 0; i < OZ_RING; ++i)
         {
             mbar_init(&full[i], 1);
-            mbar_init(&empty[i], 2);  // one commit from each MMA issuer
+            mbar_init(&empty[i], 1);
+        }
+        for (int u = 0; u < OZ_NPHASE; ++u)
+        {
+            mbar_init(&pfull[u], 1);
         }
         for (int u = 0; u < OZ_NACC; ++u)
         {
-            mbar_init(&tfull[u], 1);
             mbar_init(&tempty[u], 2 * OZ_EPI_WARPS);
         }
-        mbar_init(drain, 2);
+        mbar_init(drain, 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -427,7 +514,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
                 for (int kb = 0; ok && kb < p.nkb; ++kb)
                 {
                     const int xa = p.a_col0 + kb * OZ_KB, xb = p.b_col0 + kb * OZ_KB;
-                    for (int g = 0; ok && g < G; ++g)
+                    for (int g = G - 1; ok && g >= 0; --g)
                     {
                         // slot n % OZ_RING takes A_g and B_g; one barrier counts both
                         const int slot = n % OZ_RING;
@@ -457,94 +544,131 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
             }
         }
     }
-    else if (warp == 1 || warp == 2)
+    else if (warp == 2 && leader)
     {
-        if (lane == 0 && leader)
+        // ---------------- scout (leader) ----------------
+        // Waits for what each unit needs -- its accumulator read, and for a
+        // block's first unit the block's digit planes -- and passes it on to
+        // the issuer's warp through a hardware barrier.  The MMAs read their
+        // operands at three quarters of the shared memory's bandwidth, so a
+        // test of a shared-memory barrier takes 110 to 240 cycles beside them;
+        // in the issuing thread, which runs in step with the tensor core, each
+        // of these would be a gap.  The scout is at most four units ahead (it
+        // waits for the accumulator of the unit four back), so no barrier is
+        // arrived on twice; after a wait that gave up it only keeps pace.
+        int n = 0, nu = 0;
+        bool ok = true;
+        for (int t = pair; t < p.ntiles; t += npairs)
         {
-            // ---------------- MMA issuers (leader only, two threads) ----------------
-            // An issuing thread runs in step with the tensor core (an MMA issue
-            // returns about when the previous one completes), and a barrier
-            // test in that thread costs a shared-memory round trip, which is
-            // slow while the tensor core streams its operands; the tensor core
-            // would sit idle for it.  Two threads (warps 1 and 2) therefore
-            // issue: groups of even global index from one, odd from the other
-            // (so each owns two of the four accumulators), and while one waits
-            // the other's MMAs keep the tensor core busy.  Before a group a
-            // thread waits for its accumulator and for the digit planes of
-            // the block it has not seen yet; after the block both threads
-            // commit to each slot's empty barrier (count 2).  Descriptors
-            // advance from the ring bases (a slot is OZ_A_BYTES / 16 or
-            // OZ_B_BYTES / 16 units of the descriptor's address field).
-            const int me = warp - 1;
-            const uint64_t adesc0 = sw128_desc(smem_u32(aring));
-            const uint64_t bdesc0 = sw128_desc(smem_u32(bring));
-            int n = 0, nu = 0;
-            bool ok = true;
-            for (int t = pair; ok && t < p.ntiles; t += npairs)
+            for (int kb = 0; kb < p.nkb; ++kb, n += G)
             {
-                for (int kb = 0; ok && kb < p.nkb; ++kb)
+                for (int j = 0; j < G; ++j, ++nu)
                 {
-                    const int s0 = n % OZ_RING;  // slot of this block's plane 0
-                    int seen = -1;               // planes of this block this thread has waited for
-                    for (int g = 0; ok && g < G; ++g, ++nu)
+                    const int u = nu % OZ_NACC;
+                    const bool was = ok;
+                    // lane 31 the accumulator, lanes 0 .. G - 1 a plane each, at once
+                    if (ok && lane == 31 && nu >= OZ_NACC)
                     {
-                        if ((nu & 1) != me)
-                        {
-                            continue;
-                        }
-                        const int u = nu % OZ_NACC;
-                        if (nu >= OZ_NACC && !mbar_wait(&tempty[u], ((nu / OZ_NACC) & 1u) ^ 1u, abort_flag))
-                        {
-                            ok = false;
-                            break;
-                        }
-                        for (int pl = seen + 1; ok && pl <= g; ++pl)
-                        {
-                            const int ni = n + pl;
-                            ok = mbar_wait(&full[ni % OZ_RING], (ni / OZ_RING) & 1u, abort_flag);
-                        }
-                        if (!ok)
-                        {
-                            break;
-                        }
-                        seen = g;
-                        tc_fence_after();
-                        const uint32_t d = tmem_base + static_cast<uint32_t>(u * 128);
-                        int aslot = s0;      // slot of A_pa
-                        int bslot = s0 + g;  // slot of B_{g-pa}
-                        bslot -= bslot >= OZ_RING ? OZ_RING : 0;
-                        for (int pa = 0; pa <= g; ++pa)  // A plane pa against B plane g - pa
-                        {
-                            const uint64_t adesc = adesc0 + static_cast<uint64_t>(aslot * (OZ_A_BYTES >> 4));
-                            const uint64_t bdesc = bdesc0 + static_cast<uint64_t>(bslot * (OZ_B_BYTES >> 4));
-#pragma unroll
-                            for (int kk = 0; kk < 4; ++kk)
-                            {
-                                // 32 bytes of K per instruction: advance the start address by 2 x 16 B
-                                mma_i8_pair(d, adesc + 2 * kk, bdesc + 2 * kk, (pa | kk) != 0 ? 1u : 0u);
-                            }
-                            aslot = aslot + 1 == OZ_RING ? 0 : aslot + 1;
-                            bslot = bslot == 0 ? OZ_RING - 1 : bslot - 1;
-                        }
-                        mma_commit_pair_both(&tfull[u]);
+                        ok = mbar_wait(&tempty[u], ((nu / OZ_NACC) & 1u) ^ 1u, abort_flag);
                     }
-                    if (!ok)
+                    if (ok && j == 0 && lane < G)
                     {
-                        break;
+                        ok = mbar_wait(&full[(n + lane) % OZ_RING], ((n + lane) / OZ_RING) & 1u, abort_flag);
                     }
-                    // a slot is free once both threads' MMAs of this block complete
-                    for (int pa = 0; pa < G; ++pa)
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (ok)
                     {
-                        const int sl = s0 + pa;
-                        mma_commit_pair_both(&empty[sl >= OZ_RING ? sl - OZ_RING : sl]);
+                        scout_arrive(u);
+                        continue;
                     }
-                    n += G;
+                    if (was)
+                    {
+                        // a millisecond for the issuer to take what has been
+                        // signalled (it waits for nothing else)
+                        const unsigned long long t0 = global_ns();
+                        while (global_ns() - t0 < 1000000ull)
+                        {
+                            __nanosleep(1000);
+                        }
+                        __syncwarp();
+                    }
+                    scout_sync(u);
                 }
             }
-            // drain (count 2): completes once every MMA both threads issued has completed
-            mma_commit_pair_local(drain);
-            mbar_wait(drain, 0u, abort_flag);
         }
+    }
+    else if (warp == 1 && leader)
+    {
+        // ---------------- MMA issuer (leader, one lane) ----------------
+        // Descending groups, the largest first: the epilogue reads it and the
+        // next while the others are multiplied.  Plane q is last read by group q, so its
+        // slot is free long before the block's end, and the next block's
+        // planes, loaded in the same order, find it.  Everything between two MMAs
+        // is a gap (an issue returns about when the MMA before has completed),
+        // so a block's MMAs are unrolled over descriptors made before it (1986
+        // -> 2025 TOP/s at 8192^3, 5 groups).  Descriptors advance from
+        // the ring bases (a slot is OZ_A_BYTES / 16 or OZ_B_BYTES / 16 units of
+        // the descriptor's address field).
+        const uint64_t adesc0 = sw128_desc(smem_u32(aring));
+        const uint64_t bdesc0 = sw128_desc(smem_u32(bring));
+        int s0 = 0, nu = 0, np = 0;  // slot of the block's plane G - 1, units, phases
+        for (int t = pair; t < p.ntiles; t += npairs)
+        {
+            for (int kb = 0; kb < p.nkb; ++kb)
+            {
+                // the planes' slots and descriptors, before the block's first MMA
+                int slot[G];
+                uint64_t adesc[G], bdesc[G];
+#pragma unroll
+                for (int pl = 0; pl < G; ++pl)
+                {
+                    slot[pl] = s0 + G - 1 - pl;
+                    slot[pl] -= slot[pl] >= OZ_RING ? OZ_RING : 0;
+                    adesc[pl] = adesc0 + static_cast<uint64_t>(slot[pl] * (OZ_A_BYTES >> 4));
+                    bdesc[pl] = bdesc0 + static_cast<uint64_t>(slot[pl] * (OZ_B_BYTES >> 4));
+                }
+#pragma unroll
+                for (int j = 0; j < G; ++j, ++nu)
+                {
+                    const int g = G - 1 - j;
+                    const int u = nu % OZ_NACC;
+                    scout_sync(u);
+                    if (lane == 0)
+                    {
+                        tc_fence_after();
+                        const uint32_t d = tmem_base + static_cast<uint32_t>(u * 128);
+#pragma unroll
+                        for (int pa = 0; pa <= g; ++pa)  // A plane pa against B plane g - pa
+                        {
+#pragma unroll
+                            for (int kk = 0; kk < OZ_KB / 32; ++kk)
+                            {
+                                // 32 bytes of K per instruction: advance the start address by 2 x 16 B
+                                mma_i8_pair(d, adesc[pa] + 2 * kk, bdesc[g - pa] + 2 * kk, (pa | kk) != 0 ? 1u : 0u);
+                            }
+                        }
+                        mma_commit_pair_both(&empty[slot[g]]);
+                        if (phase_ends(j, G))
+                        {
+                            mma_commit_pair_both(&pfull[np % OZ_NPHASE]);
+                        }
+                    }
+                    __syncwarp();
+                    np += phase_ends(j, G) ? 1 : 0;
+                }
+                s0 += G;
+                s0 -= s0 >= OZ_RING ? OZ_RING : 0;
+            }
+        }
+        if (lane == 0)
+        {
+            // drain: completes once every MMA issued has completed (waited for
+            // after an abort too)
+            volatile int gave_up = 0;
+            mma_commit_pair_local(drain);
+            mbar_wait(drain, 0u, &gave_up);
+        }
+        __syncwarp();
     }
     else if (warp >= 4)
     {
@@ -553,8 +677,8 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
         const int ew = warp - 4;
         const int q = warp & 3;  // TMEM lane quarter this warp may access
         const int h = ew >> 2;   // column half
-        int nu = 0;
-        bool ok = true;
+        int nu = 0, np = 0;
+        bool ok = true, there = false;
         for (int t = pair; ok && t < p.ntiles; t += npairs)
         {
             int mp, n0;
@@ -570,6 +694,20 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
             {
                 acc[j] = 0.0;
             }
+            if (p.beta && rvalid)
+            {
+                // the row's C values towards L2 while the products run
+                const double *crow = p.C + static_cast<int64_t>(row) * p.ldc;
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                {
+                    const int col = n0 + h * 64 + 16 * c;
+                    if (col < p.N && (!p.lower || col <= row))
+                    {
+                        asm volatile("prefetch.global.L2 [%0];" ::"l"(crow + col));
+                    }
+                }
+            }
             int ea_next = earow[0], eb_next = ebblk[0];
             for (int kb = 0; ok && kb < p.nkb; ++kb)
             {
@@ -582,18 +720,162 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
                     eb_next = ebblk[kb + 1];
                 }
                 const bool bad = ea == OZ_BAD_EXP || eb == OZ_BAD_EXP;
-                // groups in pairs (g, g + 1): OZ_BASE P_g + P_{g+1} is exact in int32
-                // (at most 2,112,012,032 for the pair (4, 5), the largest), so one
-                // conversion and one FMA serve both
-                for (int g = 0; g < G; g += 2)
+                if constexpr (SUM)
                 {
-                    const bool two = g + 1 < G;
+                    const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(q * 32) << 16) +
+                                               static_cast<uint32_t>(h * 64);
+                    const double sc = bad ? __longlong_as_double(0x7ff8000000000000ll)
+                                          : pow2(ea + eb - 12) * p.wpow[G - 1];
+                    // Has phase np completed?  Its test is issued before the last
+                    // products of the phase before it, so that a phase which is
+                    // there by then costs no wait; else one lane polls (the others'
+                    // polls would take shared-memory bandwidth from the MMAs).
+                    auto phase_test = [&]()
+                    { return mbar_test_wait(&pfull[np % OZ_NPHASE], (np / OZ_NPHASE) & 1u); };
+                    auto phase_ready = [&]()
+                    {
+                        if (!__all_sync(0xffffffffu, there))
+                        {
+                            if (lane == 0)
+                            {
+                                ok = mbar_wait(&pfull[np % OZ_NPHASE], (np / OZ_NPHASE) & 1u, abort_flag);
+                            }
+                            ok = __all_sync(0xffffffffu, ok);
+                        }
+                        ++np;
+                        return ok;
+                    };
+                    auto unit_base = [&](int j)
+                    { return lane_base + static_cast<uint32_t>(((nu + j) % OZ_NACC) * 128); };
+                    // every load of units j0 .. j1 - 1 has arrived: the MMAs may reuse them
+                    auto release = [&](int j0, int j1)
+                    {
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0)
+                        {
+                            for (int j = j0; j < j1; ++j)
+                            {
+                                mbar_arrive_remote(map_to_rank(&tempty[(nu + j) % OZ_NACC], 0));
+                            }
+                        }
+                    };
+                    // the two highest groups, G - 1 (unit 0) and G - 2 (unit 1), the
+                    // block's longest: 254 P_{G-2} + P_{G-1} kept in 64 registers
+                    if (!phase_ready())
+                    {
+                        break;
+                    }
+                    tc_fence_after();
+                    int32_t low[64];
+                    {
+                        const uint32_t t0 = unit_base(0), t1 = unit_base(1);
+                        int32_t hi[2][16], lo[2][16];
+                        tmem_ld16_i(t0, lo[0]);
+                        tmem_ld16_i(t1, hi[0]);
+#pragma unroll
+                        for (int c = 0; c < 4; ++c)
+                        {
+                            tmem_ld_wait();
+                            regs_loaded(lo[c & 1]);
+                            regs_loaded(hi[c & 1]);
+                            if (c < 3)
+                            {
+                                tmem_ld16_i(t0 + (c + 1) * 16, lo[(c + 1) & 1]);
+                                tmem_ld16_i(t1 + (c + 1) * 16, hi[(c + 1) & 1]);
+                            }
+                            else
+                            {
+                                release(0, 2);
+                                there = phase_test();
+                            }
+#pragma unroll
+                            for (int k = 0; k < 16; ++k)
+                            {
+                                low[16 * c + k] = hi[c & 1][k] * OZ_IBASE + lo[c & 1][k];
+                            }
+                        }
+                    }
+                    // the other groups, 8 columns at a time, and the block's sum
+                    // into the accumulators; meanwhile the MMAs work on the next
+                    // block's longest group.  The next columns are requested
+                    // early once enough of `low` is used up to hold them.
+                    if (!phase_ready())
+                    {
+                        break;
+                    }
+                    tc_fence_after();
+                    {
+                        constexpr int U = G - 2;      // units left: groups U - 1 .. 0
+                        constexpr int AHEAD_FROM = U == 3 ? 2 : 0;
+                        uint32_t tb[U];
+#pragma unroll
+                        for (int j = 0; j < U; ++j)
+                        {
+                            tb[j] = unit_base(G - 1 - j);  // group j
+                        }
+                        int32_t v[2][U][8];
+#pragma unroll
+                        for (int c = 0; c < 8; ++c)
+                        {
+                            if (c <= AHEAD_FROM)
+                            {
+#pragma unroll
+                                for (int j = 0; j < U; ++j)
+                                {
+                                    tmem_ld8_i(tb[j] + 8 * c, v[c & 1][j]);
+                                }
+                            }
+                            tmem_ld_wait();
+#pragma unroll
+                            for (int j = 0; j < U; ++j)
+                            {
+                                regs_loaded(v[c & 1][j]);
+                            }
+                            if (c >= AHEAD_FROM && c < 7)
+                            {
+#pragma unroll
+                                for (int j = 0; j < U; ++j)
+                                {
+                                    tmem_ld8_i(tb[j] + 8 * (c + 1), v[(c + 1) & 1][j]);
+                                }
+                            }
+                            if (c == 7)
+                            {
+                                release(2, G);
+                                there = phase_test();
+                            }
+#pragma unroll
+                            for (int k = 0; k < 8; ++k)
+                            {
+                                const double x = sum_of_groups<G>(v[c & 1][0][k], U > 1 ? v[c & 1][U > 1 ? 1 : 0][k] : 0,
+                                                                   U > 2 ? v[c & 1][U > 2 ? 2 : 0][k] : 0,
+                                                                   low[8 * c + k]);
+                                acc[8 * c + k] = fma(x, sc, acc[8 * c + k]);
+                            }
+                        }
+                    }
+                    nu += G;
+                }
+                // groups in pairs (g, g - 1) from the top: OZ_BASE P_{g-1} + P_g is
+                // exact in int32, so one conversion and one FMA serve both
+                for (int j = 0; !SUM && j < G; ++np)
+                {
+                    const int g = G - 1 - j;
+                    const bool two = !phase_ends(j, G);
+                    j += two ? 2 : 1;
                     const int u0 = nu % OZ_NACC;
                     const int u1 = (nu + 1) % OZ_NACC;
-                    if (!mbar_wait(&tfull[u0], (nu / OZ_NACC) & 1u, abort_flag) ||
-                        (two && !mbar_wait(&tfull[u1], ((nu + 1) / OZ_NACC) & 1u, abort_flag)))
+                    if (!__all_sync(0xffffffffu, there))
                     {
-                        ok = false;
+                        if (lane == 0)
+                        {
+                            ok = mbar_wait(&pfull[np % OZ_NPHASE], (np / OZ_NPHASE) & 1u, abort_flag);
+                        }
+                        ok = __all_sync(0xffffffffu, ok);
+                    }
+                    if (!ok)
+                    {
                         break;
                     }
                     tc_fence_after();
@@ -601,9 +883,8 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
                                                static_cast<uint32_t>(h * 64);
                     const uint32_t t0 = lane_base + static_cast<uint32_t>(u0 * 128);
                     const uint32_t t1 = lane_base + static_cast<uint32_t>(u1 * 128);
-                    // a last unpaired group counts as OZ_BASE P_g + 0 at the pair's scale
                     const double sc = bad ? __longlong_as_double(0x7ff8000000000000ll)
-                                          : pow2(ea + eb - 12) * p.wpow[g + 1];
+                                          : pow2(ea + eb - 12) * p.wpow[g];
                     // 16 columns of each group at a time, double-buffered: the next
                     // chunk's tensor-memory loads are in flight while this chunk converts
                     auto chunk = [&](int32_t(&v)[16], int32_t(&w)[16], int32_t(&vn)[16], int32_t(&wn)[16], int c)
@@ -640,11 +921,12 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
                                     mbar_arrive_remote(map_to_rank(&tempty[u1], 0));
                                 }
                             }
+                            there = mbar_test_wait(&pfull[(np + 1) % OZ_NPHASE], ((np + 1) / OZ_NPHASE) & 1u);
                         }
 #pragma unroll
                         for (int k = 0; k < 16; ++k)
                         {
-                            acc[c * 16 + k] = fma(i2d(v[k] * OZ_IBASE + w[k]), sc, acc[c * 16 + k]);
+                            acc[c * 16 + k] = fma(i2d(w[k] * OZ_IBASE + v[k]), sc, acc[c * 16 + k]);
                         }
                     };
                     int32_t va[16], wa[16], vb[16], wb[16];
@@ -979,8 +1261,13 @@ void oz_gemm(const OzOperand &A, const OzOperand &B, const OzGemmArgs &a, cudaSt
     attr[1] = programmatic_launch_attr();
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    ensure_smem_attr(reinterpret_cast<const void *>(oz_gemm_kernel), OZ_SMEM_BYTES);
-    GPRAT_CUDA_CHECK(cudaLaunchKernelEx(&cfg, oz_gemm_kernel, A.map_a, B.map_b, k));
+    static_assert(OZ_MAX_SLICES == 7, "a kernel for each number of groups");
+    constexpr decltype(&oz_gemm_kernel<1>) kernels[] = {oz_gemm_kernel<1>, oz_gemm_kernel<2>, oz_gemm_kernel<3>,
+                                                        oz_gemm_kernel<4>, oz_gemm_kernel<5>, oz_gemm_kernel<6>,
+                                                        oz_gemm_kernel<7>};
+    const auto kern = kernels[G - 1];
+    ensure_smem_attr(reinterpret_cast<const void *>(kern), OZ_SMEM_BYTES);
+    GPRAT_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, A.map_a, B.map_b, k));
     GPRAT_LAUNCH_CHECK();
     if (timed)
     {

@@ -20,9 +20,10 @@
 // and the G = s groups of one block form one unit of int32 accumulation in
 // tensor memory (tcgen05.mma kind::i8) each; the epilogue combines two
 // groups exactly in int32 (254 P_g + P_{g+1}, at most 2,112,012,032 for
-// the largest pair (4, 5)), converts the sum exactly to FP64 and adds it
-// with its scale by one FMA, so the roundings are the digit truncation, the
-// scale 254^-(g+1) and FP64 additions.
+// the largest pair (4, 5)) or all of them exactly in 64-bit integers (3 and 5
+// groups), converts the sum exactly to FP64 and adds it with its scale by one
+// FMA, so the roundings are the digit truncation, the scale 254^-g and FP64
+// additions.
 #pragma once
 
 #include "common.cuh"

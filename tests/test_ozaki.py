@@ -198,3 +198,23 @@ def test_gemm_rejects_bad_shapes(capi):
         capi.test_oz_gemm(A, B, C, 1.0, 0.0, 6)  # K not a multiple of 128
     with pytest.raises(capi.GpratCudaError):
         capi.test_oz_gemm(np.zeros((128, 128)), np.zeros((128, 128)), C, 1.0, 0.0, 9)  # too many digits
+
+
+@pytest.mark.parametrize("G", [1, 2, 3, 4, 5, 6, 7])
+@pytest.mark.parametrize("largest", [False, True])
+def test_gemm_each_number_of_groups(capi, G, largest):
+    """Every group count over several blocks and tiles of one CTA pair (the
+    ring, the accumulators and the phases wrap), with graded rows and with
+    every digit as large as it gets, where the groups' sums are largest."""
+    M, N, K, s = 600, 200, 1280, max(3, G)
+    rng = np.random.default_rng(G)
+    if largest:
+        x = sum((63 if p == 0 else 127) * wpow(p) for p in range(s)) / 64.0
+        A = np.full((M, K), x) * np.exp2(rng.integers(-3, 4, size=(M, 1)))
+        B = np.full((N, K), -x)
+    else:
+        A, B = graded(rng, M, K), graded(rng, N, K)
+    C = np.zeros((M, N))
+    capi.test_oz_gemm(A, B, C, 1.0, 0.0, s, G, False, max_ctas=2)
+    ref, mag = np_oz_gemm(A, B, C, 1.0, 0.0, s, G)
+    assert np.all(np.abs(C - ref) <= 2.0 ** -46 * mag)
