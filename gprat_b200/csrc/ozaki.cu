@@ -40,11 +40,9 @@
 //     64 FP64 accumulators per thread.  Other G: pairs of groups, each
 //     converted and added so (at most 2,112,012,032 in int32).  The next
 //     block's exponents are loaded while a block is read.  After the tile's
-//     last unit, alpha * acc is written from the registers, 8 columns at a
-//     time, each lane its own row with 16-byte stores (beta = 1 adds to C,
-//     whose lines were sent for when the tile began; those C
-//     values are loaded first); the shared memory a staging transpose would
-//     take holds a ninth digit-plane slot instead.
+//     last unit, alpha * acc (+ C, whose lines were sent for when the tile
+//     began) is written 16 columns at a time through 4 KB of shared memory per
+//     warp, whole 128-byte lines at once.
 // What bounds it: the epilogue.  FP64 instructions take 3.2 times as long
 // while int8 MMAs stream (12 cycles a warp instruction and scheduler instead
 // of 4), and so do integer ones between them, so what counts is the FP64
@@ -52,10 +50,10 @@
 // groups is converted by itself.  One 256 x 128 x 128 block of 5 groups takes
 // 8400 cycles, of which its MMAs are 3840 (64 each); with the epilogue's
 // arithmetic left out 5400, with the integer sums alone 7100.  At 8192^3, 5
-// groups, 1785 -> 2032 TOP/s against two issuing threads that waited for the
+// groups, 1785 -> 2085 TOP/s against two issuing threads that waited for the
 // barriers themselves and three pairs per block; lower 28672^2 x 2048: 1603 ->
-// 1783; 8192 x 128 x 1920: 96.2 -> 87 us; 3 groups 1293 -> 1405.  4 groups: 1650 to
-// 1800 from run to run (before 1720).
+// 1940; 8192 x 128 x 1920: 96.2 -> 82 us; 8192 x 128 x 128: 25.6 -> 19.5 us; 3
+// groups 1293 -> 1460.  4 groups: 1680 to 1780 from run to run (before 1720).
 // Every mbarrier wait is bounded (tcgen05_ptx.cuh); a wait that gives up
 // raises the CTA's abort flag, the roles leave their loops, TMA copies in
 // flight get 200 us to land, the MMA issuer drains, TMEM is freed and the
@@ -255,12 +253,16 @@ static_assert(128 * OZ_REGS_PRODUCER + 256 * OZ_REGS_EPILOGUE <= OZ_THREADS * 16
 constexpr int OZ_EPI_WARPS = 8;
 constexpr int OZ_A_BYTES = 128 * 128;  // 128 rows x 128 digit bytes
 constexpr int OZ_B_BYTES = 64 * 128;   // this CTA's half of the 128 B rows
-constexpr int OZ_RING = 9;  // slots of one A and one B digit plane (>= s + 1: the next block's first planes load early)
+// Slots of one A and one B digit plane: >= s + 1, so that the next block's first
+// planes load early, and a power of two, so that a slot's index is a mask (9
+// slots: 2030 TOP/s at 8192^3, 5 groups; 8: 2110).
+constexpr int OZ_RING = 8;
 constexpr int OZ_NACC = 4;             // int32 accumulators of 128 TMEM columns
 constexpr int OZ_NPHASE = 4;           // barriers of the epilogue's phases, in turn
 constexpr int OZ_TMEM_COLS = OZ_NACC * 128;
+constexpr int OZ_STAGE_BYTES = 32 * 128;  // an epilogue warp's 32 rows x 16 columns on their way to or from memory
 constexpr int OZ_SMEM_BYTES =
-    1024 + OZ_RING * (OZ_A_BYTES + OZ_B_BYTES) + 512;
+    1024 + OZ_RING * (OZ_A_BYTES + OZ_B_BYTES) + OZ_EPI_WARPS * OZ_STAGE_BYTES + 512;
 static_assert(OZ_SMEM_BYTES <= 232448, "shared memory of the int8 GEMM exceeds the per-CTA limit");
 static_assert(OZ_RING >= OZ_MAX_SLICES + 1, "the ring must hold one block's planes plus one");
 // D = S32, A and B signed 8-bit, K-major, N = 128, M = 256 (CTA pair)
@@ -272,7 +274,7 @@ constexpr int OZ_GROUP_M = 8;  // row tiles per group of the non-lower tile orde
 // saves FP64 instructions enough to pay for its two widening multiplications.
 // 3 groups: 1405 TOP/s at 8192^3 against 1300 in pairs; 5: 2030 against 1800;
 // 4: 1615 against 1700, so pairs; above 5 the sum has more than 52 bits.
-constexpr bool oz_sums(int G)
+__host__ __device__ constexpr bool oz_sums(int G)
 {
     return G == 3 || G == 5;
 }
@@ -446,7 +448,8 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t *aring = smem;
     uint8_t *bring = aring + OZ_RING * OZ_A_BYTES;
-    uint64_t *full = reinterpret_cast<uint64_t *>(bring + OZ_RING * OZ_B_BYTES);
+    uint8_t *stages = bring + OZ_RING * OZ_B_BYTES;
+    uint64_t *full = reinterpret_cast<uint64_t *>(stages + OZ_EPI_WARPS * OZ_STAGE_BYTES);
     uint64_t *empty = full + OZ_RING;
     uint64_t *pfull = empty + OZ_RING;
     uint64_t *tempty = pfull + OZ_NPHASE;
@@ -503,7 +506,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
             // ---------------- TMA producer (both CTAs) ----------------
             asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmA)) : "memory");
             asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmB)) : "memory");
-            int n = 0;  // digit-plane pairs loaded
+            uint32_t n = 0;  // digit-plane pairs loaded
             bool ok = true;
             for (int t = pair; ok && t < p.ntiles; t += npairs)
             {
@@ -556,7 +559,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
         // of these would be a gap.  The scout is at most four units ahead (it
         // waits for the accumulator of the unit four back), so no barrier is
         // arrived on twice; after a wait that gave up it only keeps pace.
-        int n = 0, nu = 0;
+        uint32_t n = 0, nu = 0;
         bool ok = true;
         for (int t = pair; t < p.ntiles; t += npairs)
         {
@@ -611,7 +614,8 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
         // the descriptor's address field).
         const uint64_t adesc0 = sw128_desc(smem_u32(aring));
         const uint64_t bdesc0 = sw128_desc(smem_u32(bring));
-        int s0 = 0, nu = 0, np = 0;  // slot of the block's plane G - 1, units, phases
+        int s0 = 0;  // slot of the block's plane G - 1
+        uint32_t nu = 0, np = 0;  // units, phases
         for (int t = pair; t < p.ntiles; t += npairs)
         {
             for (int kb = 0; kb < p.nkb; ++kb)
@@ -677,7 +681,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
         const int ew = warp - 4;
         const int q = warp & 3;  // TMEM lane quarter this warp may access
         const int h = ew >> 2;   // column half
-        int nu = 0, np = 0;
+        uint32_t nu = 0, np = 0;
         bool ok = true, there = false;
         for (int t = pair; ok && t < p.ntiles; t += npairs)
         {
@@ -954,67 +958,77 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
             {
                 break;
             }
-            // ---- write alpha * acc: each lane its own row, 8 columns at a time ----
-            // 16-byte stores straight from the registers (no shared-memory
-            // staging, which leaves its space to the digit-plane ring); with
-            // beta = 1 the 8 columns' C values are loaded first.
+            // ---- write alpha * acc, 16 columns at a time ----
+            // Through the warp's 4 KB of shared memory (16-byte units, swizzled
+            // by the row), so that 8 lanes move 128 consecutive bytes of a row:
+            // with each lane at its own row a tile took 25,000 cycles, most of
+            // them waiting for the C values (beta = 1).
             double sq = 0.0;
-            double *crow = p.C + static_cast<int64_t>(rvalid ? row : 0) * p.ldc;
+            double2 *stage = reinterpret_cast<double2 *>(stages + ew * OZ_STAGE_BYTES);
 #pragma unroll
-            for (int c = 0; c < 8; ++c)
+            for (int c = 0; c < 4; ++c)
             {
-                const int col0 = n0 + h * 64 + c * 8;
+                const int col0 = n0 + h * 64 + c * 16;
                 // warp-uniform: chunk right of C, below C, or (lower) above the diagonal for all rows
                 if (col0 >= p.N || row0w >= p.M || (p.lower && col0 > row0w + 31))
                 {
                     continue;
                 }
-                double2 cold[4];
+                const int gc = col0 + 2 * (lane & 7);    // this lane's two columns of rows row0w + lane / 8 + 4 i
+                const int gr = row0w + (lane >> 3);
+                double *cptr = p.C + static_cast<int64_t>(gr) * p.ldc + gc;
+                double2 cold[8];
 #pragma unroll
-                for (int j = 0; j < 4; ++j)
+                for (int i = 0; i < 8; ++i)
                 {
-                    const int gc = col0 + 2 * j;
-                    const bool full = rvalid && gc + 1 < p.N && (!p.lower || gc + 1 <= row);
-                    cold[j] = (p.beta && full) ? *reinterpret_cast<const double2 *>(crow + gc) : make_double2(0.0, 0.0);
+                    const int r = gr + 4 * i;
+                    const bool full = r < p.M && gc + 1 < p.N && (!p.lower || gc + 1 <= r);
+                    cold[i] = (p.beta && full) ? *reinterpret_cast<const double2 *>(cptr + 4 * i * p.ldc)
+                                               : make_double2(0.0, 0.0);
                 }
 #pragma unroll
-                for (int j = 0; j < 4; ++j)
+                for (int u = 0; u < 8; ++u)
                 {
-                    const int gc = col0 + 2 * j;
-                    const double x = p.alpha * acc[c * 8 + 2 * j];
-                    const double y = p.alpha * acc[c * 8 + 2 * j + 1];
+                    const double x = p.alpha * acc[c * 16 + 2 * u];
+                    const double y = p.alpha * acc[c * 16 + 2 * u + 1];
                     if (p.rowsq != nullptr && rvalid)
                     {
-                        if (gc < p.N)
+                        if (col0 + 2 * u < p.N)
                         {
                             sq += x * x;
                         }
-                        if (gc + 1 < p.N)
+                        if (col0 + 2 * u + 1 < p.N)
                         {
                             sq += y * y;
                         }
                     }
-                    if (!rvalid)
-                    {
-                        continue;
-                    }
-                    const bool ok0 = gc < p.N && (!p.lower || gc <= row);
-                    const bool ok1 = gc + 1 < p.N && (!p.lower || gc + 1 <= row);
+                    stage[lane * 8 + (u ^ (lane & 7))] = make_double2(x, y);
+                }
+                __syncwarp();
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                {
+                    const int rr = (lane >> 3) + 4 * i;
+                    const int r = row0w + rr;
+                    double2 o = stage[rr * 8 + ((lane & 7) ^ (rr & 7))];
+                    const bool ok0 = r < p.M && gc < p.N && (!p.lower || gc <= r);
+                    const bool ok1 = r < p.M && gc + 1 < p.N && (!p.lower || gc + 1 <= r);
+                    double *dst = cptr + 4 * i * p.ldc;
                     if (ok0 && ok1)
                     {
-                        double2 o = make_double2(x, y);
                         if (p.beta)
                         {
-                            o.x += cold[j].x;
-                            o.y += cold[j].y;
+                            o.x += cold[i].x;
+                            o.y += cold[i].y;
                         }
-                        *reinterpret_cast<double2 *>(crow + gc) = o;
+                        *reinterpret_cast<double2 *>(dst) = o;
                     }
                     else if (ok0)
                     {
-                        crow[gc] = p.beta ? crow[gc] + x : x;
+                        *dst = p.beta ? *dst + o.x : o.x;
                     }
                 }
+                __syncwarp();
             }
             __syncwarp();
             if (p.rowsq != nullptr && rvalid)
