@@ -95,6 +95,8 @@ def _load() -> ctypes.CDLL:
     lib.gprat_cu_test_oz_gemm.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_int, _dp, _dp, _dp, ctypes.c_double,
                                           ctypes.c_double, ctypes.c_int, ctypes.c_int, ctypes.c_int, _dp,
                                           ctypes.c_int]
+    lib.gprat_cu_test_oz_emit.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_int, _dp, _dp, _dp, ctypes.c_double,
+                                          ctypes.c_int, ctypes.c_int, ctypes.c_int, _i8p, _i32p, _i8p, _i32p]
     lib.gprat_cu_steps_csv.argtypes = [ctypes.c_char_p, _i64, _i64p]
     lib.gprat_cu_server_create.argtypes = [ctypes.c_int, _i64, ctypes.c_int, ctypes.POINTER(_vp)]
     lib.gprat_cu_server_destroy.argtypes = [_vp]
@@ -268,6 +270,24 @@ def test_oz_gemm(A: np.ndarray, B: np.ndarray, C: np.ndarray, alpha: float, beta
     rp = _p(rowsq) if rowsq is not None else None
     check(lib.gprat_cu_test_oz_gemm(M, N, K, _p(A), _p(B), _p(C), float(alpha), float(beta), int(bool(lower)),
                                     int(s), int(groups), rp, int(max_ctas)))
+
+
+def test_oz_emit(A: np.ndarray, B: np.ndarray, C: np.ndarray, beta: float, s: int, emit_from: int,
+                 store_rows: int) -> Tuple[np.ndarray, np.ndarray, np.ndarray, np.ndarray]:
+    """C = beta*C - A B^T in place as test_oz_gemm; also returns the digits
+    that the same launch writes of C's first 128 columns from row emit_from
+    on: (row digits, row exponents, block digits, block exponents).  Rows from
+    store_rows on of these columns are not written to C."""
+    M, K = A.shape
+    N = B.shape[0]
+    rows = M - emit_from
+    i8, i32 = ctypes.POINTER(ctypes.c_int8), ctypes.POINTER(ctypes.c_int32)
+    rd, bd = np.empty((s, rows, 128), dtype=np.int8), np.empty((s, rows, 128), dtype=np.int8)
+    re, be = np.empty((rows, 1), dtype=np.int32), np.empty(((rows + 127) // 128, 1), dtype=np.int32)
+    check(lib.gprat_cu_test_oz_emit(M, N, K, _p(A), _p(B), _p(C), float(beta), int(s), int(emit_from),
+                                    int(store_rows), rd.ctypes.data_as(i8), re.ctypes.data_as(i32),
+                                    bd.ctypes.data_as(i8), be.ctypes.data_as(i32)))
+    return rd, re, bd, be
 
 
 def _arr(a) -> np.ndarray:

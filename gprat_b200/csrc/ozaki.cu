@@ -100,13 +100,27 @@ __device__ __forceinline__ int exp_of(double vmax, bool bad)
     return e < -960 ? OZ_ZERO_EXP : e;
 }
 
+// The leading balanced base-254 digit of t, and t <- 254 (t - digit): y holds
+// the digit in its low word, 254 digit is exact from y by one FMA, and the next
+// t is rounded once, as (t - digit) 254 would be (t - digit is exact).
+__device__ __forceinline__ uint32_t next_digit(double &t)
+{
+    const double y = __dadd_rn(t, RND);
+    t = __fma_rn(t, OZ_BASE, __fma_rn(y, -OZ_BASE, OZ_BASE * RND));
+    return static_cast<uint32_t>(__double2loint(y)) & 0xffu;
+}
+
+__device__ __forceinline__ double digit_scale(int e)
+{
+    return e == OZ_ZERO_EXP || e == OZ_BAD_EXP ? 0.0 : pow2(6 - e);
+}
+
 // S digit planes of 4 consecutive values (4 bytes per plane at out + p * plane)
 template <int S>
 __device__ __forceinline__ void write_digits(const double v[4], int e, int8_t *out, int64_t plane)
 {
     double t[4];
-    const bool zero = (e == OZ_ZERO_EXP || e == OZ_BAD_EXP);
-    const double sc = zero ? 0.0 : pow2(6 - e);
+    const double sc = digit_scale(e);
 #pragma unroll
     for (int i = 0; i < 4; ++i)
     {
@@ -119,13 +133,35 @@ __device__ __forceinline__ void write_digits(const double v[4], int e, int8_t *o
 #pragma unroll
         for (int i = 0; i < 4; ++i)
         {
-            const double y = __dadd_rn(t[i], RND);
-            const int d = __double2loint(y);
-            const double r = __dsub_rn(y, RND);
-            t[i] = __dmul_rn(__dsub_rn(t[i], r), OZ_BASE);
-            word |= (static_cast<uint32_t>(d) & 0xffu) << (8 * i);
+            word |= next_digit(t[i]) << (8 * i);
         }
         *reinterpret_cast<uint32_t *>(out + p * plane) = word;
+    }
+}
+
+// S digit planes of an epilogue thread's 64 values (64 bytes per plane)
+__device__ __forceinline__ void write_row_digits(const double (&v)[64], int e, int8_t *out, int64_t plane, int S)
+{
+    const double sc = digit_scale(e);
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+    {
+        double t[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+        {
+            t[i] = __dmul_rn(v[16 * c + i], sc);
+        }
+        for (int p = 0; p < S; ++p)
+        {
+            uint32_t w[4] = { 0, 0, 0, 0 };
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+            {
+                w[i >> 2] |= next_digit(t[i]) << (8 * (i & 3));
+            }
+            *reinterpret_cast<uint4 *>(out + p * plane + 16 * c) = make_uint4(w[0], w[1], w[2], w[3]);
+        }
     }
 }
 
@@ -317,9 +353,14 @@ struct OzKernelArgs
     double *rowsq;
     int64_t rowsq_half;
     DeviceStatus *status;
-    int groups;
     int tiles_m, tiles_n, ntiles;
     double wpow[OZ_MAX_SLICES + 1];  // wpow[j] = 1 / OZ_BASE^j
+    // digits of C's first 128 columns (emit_s planes; 0: none)
+    int emit_s, emit_from, emit_row0, emit_kb, store_rows;
+    int8_t *rdig, *bdig;
+    int32_t *rexp, *bexp;
+    int64_t rld, rplane, bld, bplane;
+    int rldE, bldE;
 };
 
 __device__ __forceinline__ void tma_load_3d_pair(void *dst, const CUtensorMap *map, uint32_t leader_bar, int x, int y,
@@ -454,7 +495,8 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     uint64_t *pfull = empty + OZ_RING;
     uint64_t *tempty = pfull + OZ_NPHASE;
     uint64_t *drain = tempty + OZ_NACC;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(drain + 1);
+    uint64_t *xfull = drain + 1;  // the epilogue warps' exchange
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(xfull + 1);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5;
@@ -481,6 +523,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
             mbar_init(&tempty[u], 2 * OZ_EPI_WARPS);
         }
         mbar_init(drain, 1);
+        mbar_init(xfull, OZ_EPI_WARPS);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -681,7 +724,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
         const int ew = warp - 4;
         const int q = warp & 3;  // TMEM lane quarter this warp may access
         const int h = ew >> 2;   // column half
-        uint32_t nu = 0, np = 0;
+        uint32_t nu = 0, np = 0, nx = 0;
         bool ok = true, there = false;
         for (int t = pair; ok && t < p.ntiles; t += npairs)
         {
@@ -965,58 +1008,180 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
             // them waiting for the C values (beta = 1).
             double sq = 0.0;
             double2 *stage = reinterpret_cast<double2 *>(stages + ew * OZ_STAGE_BYTES);
+            const int cl = lane & 7, rl = lane >> 3;  // this lane moves columns 2 cl, 2 cl + 1 of rows rl + 4 i
+            double alpha = p.alpha;
+            bool beta = p.beta != 0;
+            int mst = p.M;  // rows written
+            if (p.emit_s != 0 && n0 == 0)
+            {
+                // C's new values into the registers, each lane its own row, and
+                // their digits from there: the next product's operand without
+                // writing C, reading it again and another launch
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                {
+                    if (beta)
+                    {
+                        const double *cptr = p.C + static_cast<int64_t>(row0w + rl) * p.ldc + h * 64 + c * 16 + 2 * cl;
+                        double2 cold[8];
+#pragma unroll
+                        for (int i = 0; i < 8; ++i)
+                        {
+                            cold[i] = row0w + rl + 4 * i < p.M ? *reinterpret_cast<const double2 *>(cptr + 4 * i * p.ldc)
+                                                               : make_double2(0.0, 0.0);
+                        }
+#pragma unroll
+                        for (int i = 0; i < 8; ++i)
+                        {
+                            const int rr = rl + 4 * i;
+                            stage[rr * 8 + (cl ^ (rr & 7))] = cold[i];
+                        }
+                        __syncwarp();
+                    }
+#pragma unroll
+                    for (int u = 0; u < 8; ++u)
+                    {
+                        const double2 o = beta ? stage[lane * 8 + (u ^ (lane & 7))] : make_double2(0.0, 0.0);
+                        double &x = acc[c * 16 + 2 * u], &y = acc[c * 16 + 2 * u + 1];
+                        x = __dmul_rn(alpha, x);
+                        y = __dmul_rn(alpha, y);
+                        x = beta ? __dadd_rn(x, o.x) : x;
+                        y = beta ? __dadd_rn(y, o.y) : y;
+                    }
+                    __syncwarp();
+                }
+                alpha = 1.0;
+                beta = false;
+                mst = min(mst, p.store_rows);
+                // the row's maximum (infinity if a value is not finite), shared with
+                // the warp that holds its other half, and the CTA's
+                const bool emits = rvalid && row >= p.emit_from;
+                double m = 0.0;
+                bool nonfinite = false;
+#pragma unroll
+                for (int j = 0; j < 64; ++j)
+                {
+                    const double av = fabs(acc[j]);
+                    nonfinite = nonfinite || !(av <= 1.0e308);
+                    m = fmax(m, av);
+                }
+                m = !emits ? 0.0 : nonfinite ? __longlong_as_double(0x7ff0000000000000ll) : m;
+                double *mx = reinterpret_cast<double *>(stages);
+                auto epi_sync = [&]()
+                {
+                    // the CTA's epilogue warps, with a bounded wait: one that
+                    // gave up does not come
+                    __syncwarp();
+                    if (lane == 0)
+                    {
+                        mbar_arrive_remote(map_to_rank(xfull, rank));
+                        ok = mbar_wait(xfull, nx & 1u, abort_flag);
+                    }
+                    ++nx;
+                    ok = __all_sync(0xffffffffu, ok);
+                    __syncwarp();
+                    return ok;
+                };
+                auto row_max = [&](int w) -> double & { return mx[w * (OZ_STAGE_BYTES / 8) + lane]; };
+                double wm = m;
+                if (p.bdig != nullptr)
+                {
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1)
+                    {
+                        wm = fmax(wm, __shfl_xor_sync(0xffffffffu, wm, o));
+                    }
+                }
+                row_max(ew) = m;
+                if (lane == 0)
+                {
+                    mx[ew * (OZ_STAGE_BYTES / 8) + 32] = wm;
+                }
+                if (!epi_sync())
+                {
+                    break;
+                }
+                m = fmax(m, row_max(ew ^ 4));
+                double bm = 0.0;
+#pragma unroll
+                for (int w = 0; w < OZ_EPI_WARPS; ++w)
+                {
+                    bm = fmax(bm, mx[w * (OZ_STAGE_BYTES / 8) + 32]);
+                }
+                if (!epi_sync())  // the stages are free again
+                {
+                    break;
+                }
+                const int64_t drow = p.emit_row0 + row;
+                const int64_t dcol = static_cast<int64_t>(p.emit_kb) * OZ_KB + h * 64;
+                if (p.rdig != nullptr && emits)
+                {
+                    const int e = exp_of(m, !(m <= 1.0e308));
+                    if (h == 0)
+                    {
+                        p.rexp[drow * p.rldE + p.emit_kb] = e;
+                    }
+                    write_row_digits(acc, e, p.rdig + drow * p.rld + dcol, p.rplane, p.emit_s);
+                }
+                if (p.bdig != nullptr && emits)
+                {
+                    const int e = exp_of(bm, !(bm <= 1.0e308));
+                    if (h == 0 && (row & 127) == 0)
+                    {
+                        p.bexp[drow / 128 * p.bldE + p.emit_kb] = e;
+                    }
+                    write_row_digits(acc, e, p.bdig + drow * p.bld + dcol, p.bplane, p.emit_s);
+                }
+            }
+            if (p.rowsq != nullptr && rvalid)
+            {
+#pragma unroll
+                for (int j = 0; j < 64; ++j)
+                {
+                    const double x = alpha * acc[j];
+                    sq += n0 + h * 64 + j < p.N ? x * x : 0.0;
+                }
+            }
 #pragma unroll
             for (int c = 0; c < 4; ++c)
             {
                 const int col0 = n0 + h * 64 + c * 16;
                 // warp-uniform: chunk right of C, below C, or (lower) above the diagonal for all rows
-                if (col0 >= p.N || row0w >= p.M || (p.lower && col0 > row0w + 31))
+                if (col0 >= p.N || row0w >= mst || (p.lower && col0 > row0w + 31))
                 {
                     continue;
                 }
-                const int gc = col0 + 2 * (lane & 7);    // this lane's two columns of rows row0w + lane / 8 + 4 i
-                const int gr = row0w + (lane >> 3);
+                const int gc = col0 + 2 * cl;
+                const int gr = row0w + rl;
                 double *cptr = p.C + static_cast<int64_t>(gr) * p.ldc + gc;
                 double2 cold[8];
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
                 {
                     const int r = gr + 4 * i;
-                    const bool full = r < p.M && gc + 1 < p.N && (!p.lower || gc + 1 <= r);
-                    cold[i] = (p.beta && full) ? *reinterpret_cast<const double2 *>(cptr + 4 * i * p.ldc)
-                                               : make_double2(0.0, 0.0);
+                    const bool full = r < mst && gc + 1 < p.N && (!p.lower || gc + 1 <= r);
+                    cold[i] = (beta && full) ? *reinterpret_cast<const double2 *>(cptr + 4 * i * p.ldc)
+                                             : make_double2(0.0, 0.0);
                 }
 #pragma unroll
                 for (int u = 0; u < 8; ++u)
                 {
-                    const double x = p.alpha * acc[c * 16 + 2 * u];
-                    const double y = p.alpha * acc[c * 16 + 2 * u + 1];
-                    if (p.rowsq != nullptr && rvalid)
-                    {
-                        if (col0 + 2 * u < p.N)
-                        {
-                            sq += x * x;
-                        }
-                        if (col0 + 2 * u + 1 < p.N)
-                        {
-                            sq += y * y;
-                        }
-                    }
-                    stage[lane * 8 + (u ^ (lane & 7))] = make_double2(x, y);
+                    stage[lane * 8 + (u ^ (lane & 7))] =
+                        make_double2(alpha * acc[c * 16 + 2 * u], alpha * acc[c * 16 + 2 * u + 1]);
                 }
                 __syncwarp();
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
                 {
-                    const int rr = (lane >> 3) + 4 * i;
+                    const int rr = rl + 4 * i;
                     const int r = row0w + rr;
-                    double2 o = stage[rr * 8 + ((lane & 7) ^ (rr & 7))];
-                    const bool ok0 = r < p.M && gc < p.N && (!p.lower || gc <= r);
-                    const bool ok1 = r < p.M && gc + 1 < p.N && (!p.lower || gc + 1 <= r);
+                    double2 o = stage[rr * 8 + (cl ^ (rr & 7))];
+                    const bool ok0 = r < mst && gc < p.N && (!p.lower || gc <= r);
+                    const bool ok1 = r < mst && gc + 1 < p.N && (!p.lower || gc + 1 <= r);
                     double *dst = cptr + 4 * i * p.ldc;
                     if (ok0 && ok1)
                     {
-                        if (p.beta)
+                        if (beta)
                         {
                             o.x += cold[i].x;
                             o.y += cold[i].y;
@@ -1025,7 +1190,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
                     }
                     else if (ok0)
                     {
-                        *dst = p.beta ? *dst + o.x : o.x;
+                        *dst = beta ? *dst + o.x : o.x;
                     }
                 }
                 __syncwarp();
@@ -1234,7 +1399,43 @@ void oz_gemm(const OzOperand &A, const OzOperand &B, const OzGemmArgs &a, cudaSt
     k.rowsq = a.rowsq;
     k.rowsq_half = a.rowsq_half;
     k.status = a.status;
-    k.groups = G;
+    if (a.emit_row != nullptr || a.emit_blk != nullptr)
+    {
+        for (const OzOperand *o : { a.emit_row, a.emit_blk })
+        {
+            if (o == nullptr)
+            {
+                continue;
+            }
+            if (a.lower || a.N < 128 || o->block != (o == a.emit_blk) || o->s != A.s || a.emit_col0 % OZ_KB != 0 ||
+                a.emit_from < 0 || a.emit_row0 + a.emit_from < 0 || a.emit_row0 + a.M > o->rows ||
+                a.emit_col0 + OZ_KB > o->cols || (o->block && (a.emit_row0 % 128 != 0 || a.emit_from % 128 != 0)))
+            {
+                throw Error(1, "oz_gemm: the digits of C do not fit their operand");
+            }
+        }
+        k.emit_s = A.s;
+        k.emit_from = a.emit_from;
+        k.emit_row0 = a.emit_row0;
+        k.emit_kb = a.emit_col0 / OZ_KB;
+        k.store_rows = a.store_rows;
+        if (a.emit_row != nullptr)
+        {
+            k.rdig = a.emit_row->digits;
+            k.rexp = a.emit_row->exps;
+            k.rld = a.emit_row->ld;
+            k.rplane = a.emit_row->plane;
+            k.rldE = a.emit_row->ldE;
+        }
+        if (a.emit_blk != nullptr)
+        {
+            k.bdig = a.emit_blk->digits;
+            k.bexp = a.emit_blk->exps;
+            k.bld = a.emit_blk->ld;
+            k.bplane = a.emit_blk->plane;
+            k.bldE = a.emit_blk->ldE;
+        }
+    }
     double pw = 1.0;
     for (int j = 0; j <= OZ_MAX_SLICES; ++j)
     {

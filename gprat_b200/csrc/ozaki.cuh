@@ -83,6 +83,16 @@ struct OzGemmArgs
     DeviceStatus *status;  // timeout flag if a bounded wait gives up
     int max_ctas;          // persistent grid bound (0 = every SM), leaves SMs to other streams
     int groups;            // digit groups kept, 1..s (0 = s)
+    // optional (not lower, N >= 128): the digits of C's new first 128 columns,
+    // rows [emit_from, M), as rows of emit_row and / or emit_blk (same s as A)
+    // from emit_row0 + emit_from on and columns from emit_col0 on: what
+    // oz_split would write from C.  emit_col0 a multiple of 128; for emit_blk,
+    // emit_row0 and emit_from too.  Of these columns only rows below store_rows
+    // are written to C.
+    const OzOperand *emit_row = nullptr;
+    const OzOperand *emit_blk = nullptr;
+    int emit_from = 0, emit_row0 = 0, emit_col0 = 0;
+    int store_rows = 1 << 30;
 };
 
 // C = beta C + alpha A B^T, A = rows [a_row0, a_row0 + M) of a row operand,

@@ -16,11 +16,15 @@
 // outer panels of 2048 columns (measured best at n = 32768 among 1024 to
 // 4096, with the whole pipeline timed), inside a panel left-looking over
 // 128-column blocks.  Per block column r0:
-//   update   K[r0:n, r0:r0+128] -= L[r0:n, K0:r0] L[r0:r0+128, K0:r0]^T
+//   update   K[r0:n, r0:r0+128] -= L[r0:n, K0:r0] L[r0:r0+128, K0:r0]^T, with
+//            the row digits P of the rows below the diagonal block
 //   potrf    L_kk and Linv_k in FP64 (potrf_diag)
-//   split    Linv_k -> block digits; the panel block below -> row digits
-//   solve    L[r0+128:n, r0:r0+128] = P Linv_k^T
-//   split    the solved block column -> row digits (A role) and block digits (B role)
+//   split    Linv_k -> block digits
+//   solve    L[r0+128:n, r0:r0+128] = P Linv_k^T, with its row digits (A role)
+//            and block digits (B role)
+// The products write the digits of their results themselves: as launches of
+// their own the three splits of a block column cost 80 us of n = 16384's 300,
+// and read back what had just been written.
 // The side stream (high priority) factors panel k+1 while the main stream
 // runs the trailing update of everything right of it with panel k.
 #include "gp_state.cuh"
@@ -149,7 +153,17 @@ void factor_oz(gprat_cu_gp *gp, cudaStream_t s, const std::vector<std::pair<int,
     GPRAT_CUDA_CHECK(cudaEventRecord(gp->events[0], s));
     GPRAT_CUDA_CHECK(cudaStreamWaitEvent(side, gp->events[0], 0));
 
-    // factor the block columns of panel [K0, pend) on the side stream
+    // an update of the block column r0 also writes the digits of its rows below
+    // the diagonal block, which are all the panel solve reads of them
+    auto emit_panel = [&](OzGemmArgs &a)
+    {
+        a.emit_row = &ops.P;
+        a.emit_from = NB;
+        a.emit_row0 = -NB;
+        a.store_rows = NB;
+    };
+    // factor the block columns of panel [K0, pend) on the side stream; the
+    // update before it (K0 > 0) has written the digits of its first column
     auto factor_panel = [&](int K0, int pend)
     {
         for (int r0 = K0; r0 < pend; r0 += NB)
@@ -157,9 +171,9 @@ void factor_oz(gprat_cu_gp *gp, cudaStream_t s, const std::vector<std::pair<int,
             const int k = r0 / NB;
             if (r0 > K0)
             {
-                oz_gemm(ops.LR, ops.LB, oz_args(n - r0, NB, r0 - K0, r0, K0, r0, K0, kat(gp, r0, r0), ld, -1.0, 1.0,
-                                                false, st),
-                        side);
+                OzGemmArgs a = oz_args(n - r0, NB, r0 - K0, r0, K0, r0, K0, kat(gp, r0, r0), ld, -1.0, 1.0, false, st);
+                emit_panel(a);
+                oz_gemm(ops.LR, ops.LB, a, side);
             }
             double *linv = gp->Linv.ptr + static_cast<int64_t>(k) * NB * NB;
             potrf_diag(kat(gp, r0, r0), ld, NB, r0, linv, NB, st, side);
@@ -170,10 +184,17 @@ void factor_oz(gprat_cu_gp *gp, cudaStream_t s, const std::vector<std::pair<int,
             {
                 continue;
             }
-            oz_split(kat(gp, r0 + NB, r0), ld, rows, NB, &ops.P, nullptr, 0, 0, side);
-            oz_gemm(ops.P, ops.INV,
-                    oz_args(rows, NB, NB, 0, 0, k * NB, 0, kat(gp, r0 + NB, r0), ld, 1.0, 0.0, false, st), side);
-            oz_split(kat(gp, r0 + NB, r0), ld, rows, NB, &ops.LR, &ops.LB, r0 + NB, r0, side);
+            if (r0 == 0)
+            {
+                oz_split(kat(gp, NB, 0), ld, rows, NB, &ops.P, nullptr, 0, 0, side);
+            }
+            OzGemmArgs a =
+                oz_args(rows, NB, NB, 0, 0, k * NB, 0, kat(gp, r0 + NB, r0), ld, 1.0, 0.0, false, st);
+            a.emit_row = &ops.LR;
+            a.emit_blk = &ops.LB;
+            a.emit_row0 = r0 + NB;
+            a.emit_col0 = r0;
+            oz_gemm(ops.P, ops.INV, a, side);
         }
     };
 
@@ -220,6 +241,7 @@ void factor_oz(gprat_cu_gp *gp, cudaStream_t s, const std::vector<std::pair<int,
             OzGemmArgs a = oz_args(n - pend, next_end - pend, bo, pend, K0, pend, K0, kat(gp, pend, pend), ld, -1.0,
                                    1.0, false, st);
             a.groups = fg;
+            emit_panel(a);
             oz_gemm(ops.LR, ops.LB, a, side);
         }
         factor_panel(pend, next_end);
@@ -249,20 +271,26 @@ struct OzVariance
     int max_ctas;
     cudaStream_t s;
 
-    // W[:, c0:c0+128) := W[:, c0:c0+128) Linv_k^T, row sums of squares into vacc,
-    // then the solved block's digits
+    // The digits of W[:, c0:c0+128) Linv_k^T, row sums of squares into vacc.  W
+    // itself isn't written: nothing reads a solved block but by its digits.
+    // The unsolved block's digits come from the update before it.
     void leaf(int c0) const
     {
         const int k = c0 / NB;
-        oz_split(W + c0, ld, m, NB, &WP, nullptr, 0, 0, s);
-        oz_gemm(WP, ops.INV,
-                oz_args(m, NB, NB, 0, 0, k * NB, 0, W + c0, ld, 1.0, 0.0, false, gp->status.ptr, max_ctas,
-                        gp->vacc.ptr, m),
-                s);
-        oz_split(W + c0, ld, m, NB, &WS, nullptr, 0, c0, s);
+        if (c0 == 0)
+        {
+            oz_split(W, ld, m, NB, &WP, nullptr, 0, 0, s);
+        }
+        OzGemmArgs a = oz_args(m, NB, NB, 0, 0, k * NB, 0, W + c0, ld, 1.0, 0.0, false, gp->status.ptr, max_ctas,
+                               gp->vacc.ptr, m);
+        a.emit_row = &WS;
+        a.emit_col0 = c0;
+        a.store_rows = 0;
+        oz_gemm(WP, ops.INV, a, s);
     }
 
-    // W[:, c0:c1) -= W[:, k0:k1) L[c0:c1, k0:k1)^T
+    // W[:, c0:c1) -= W[:, k0:k1) L[c0:c1, k0:k1)^T; the next call is leaf(c0),
+    // which reads the digits of the first 128 columns
     void update(int k0, int k1, int c0, int c1) const
     {
         if (k1 <= k0 || c1 <= c0)
@@ -272,6 +300,8 @@ struct OzVariance
         OzGemmArgs a = oz_args(m, c1 - c0, k1 - k0, 0, k0, c0, k0, W + c0, ld, -1.0, 1.0, false, gp->status.ptr,
                                max_ctas);
         a.groups = std::min(gp->oz_slices, gp->oz_variance_groups);
+        a.emit_row = &WP;
+        a.store_rows = 0;
         oz_gemm(WS, ops.LB, a, s);
     }
 

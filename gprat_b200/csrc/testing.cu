@@ -315,6 +315,77 @@ extern "C" int gprat_cu_test_oz_split(int rows, int cols, const double *src, int
     }
 }
 
+extern "C" int gprat_cu_test_oz_emit(int M, int N, int K, const double *A, const double *B, double *C, double beta, int s,
+                                     int emit_from, int store_rows, int8_t *rdig, int32_t *rexp, int8_t *bdig,
+                                     int32_t *bexp)
+{
+    try
+    {
+        if (A == nullptr || B == nullptr || C == nullptr || rdig == nullptr || rexp == nullptr || bdig == nullptr ||
+            bexp == nullptr || M <= 0 || N < OZ_KB || N % 2 != 0 || K <= 0 || K % OZ_KB != 0 || s < OZ_MIN_SLICES ||
+            s > OZ_MAX_SLICES || emit_from < 0 || emit_from % 128 != 0 || emit_from >= M || store_rows < 0)
+        {
+            throw Error(GPRAT_CU_ERR_INVALID_ARG, "gprat_cu_test_oz_emit: invalid arguments");
+        }
+        cudaStream_t st = nullptr;
+        const size_t bytes = static_cast<size_t>(M) * N * 8;
+        Buf dA(static_cast<size_t>(M) * K * 8), dB(static_cast<size_t>(N) * K * 8), dC(bytes);
+        GPRAT_CUDA_CHECK(cudaMemcpy(dA.p, A, static_cast<size_t>(M) * K * 8, cudaMemcpyHostToDevice));
+        GPRAT_CUDA_CHECK(cudaMemcpy(dB.p, B, static_cast<size_t>(N) * K * 8, cudaMemcpyHostToDevice));
+        GPRAT_CUDA_CHECK(cudaMemcpy(dC.p, C, bytes, cudaMemcpyHostToDevice));
+        const int rows = M - emit_from;
+        OzBuf oa(M, K, s, false), ob(N, K, s, true), er(rows, OZ_KB, s, false), eb(rows, OZ_KB, s, true);
+        oz_split(static_cast<const double *>(dA.p), K, M, K, &oa.op, nullptr, 0, 0, st);
+        oz_split(static_cast<const double *>(dB.p), K, N, K, nullptr, &ob.op, 0, 0, st);
+        Buf dStatus(sizeof(DeviceStatus));
+        GPRAT_CUDA_CHECK(cudaMemset(dStatus.p, 0, sizeof(DeviceStatus)));
+        OzGemmArgs g{};
+        g.M = M;
+        g.N = N;
+        g.K = K;
+        g.C = static_cast<double *>(dC.p);
+        g.ldc = N;
+        g.alpha = -1.0;
+        g.beta = beta;
+        g.status = static_cast<DeviceStatus *>(dStatus.p);
+        g.emit_row = &er.op;
+        g.emit_blk = &eb.op;
+        g.emit_from = emit_from;
+        g.emit_row0 = -emit_from;
+        g.store_rows = store_rows;
+        oz_gemm(oa.op, ob.op, g, st);
+        GPRAT_CUDA_CHECK(cudaStreamSynchronize(st));
+        DeviceStatus hs{};
+        GPRAT_CUDA_CHECK(cudaMemcpy(&hs, dStatus.p, sizeof(hs), cudaMemcpyDeviceToHost));
+        if (hs.timeout != 0)
+        {
+            throw Error(GPRAT_CU_ERR_TIMEOUT, "int8 GEMM: a bounded wait timed out");
+        }
+        GPRAT_CUDA_CHECK(cudaMemcpy(C, dC.p, bytes, cudaMemcpyDeviceToHost));
+        const size_t pb = static_cast<size_t>(rows) * OZ_KB;
+        for (int p = 0; p < s; ++p)
+        {
+            GPRAT_CUDA_CHECK(cudaMemcpy(rdig + p * pb, er.op.digits + p * er.op.plane, pb, cudaMemcpyDeviceToHost));
+            GPRAT_CUDA_CHECK(cudaMemcpy(bdig + p * pb, eb.op.digits + p * eb.op.plane, pb, cudaMemcpyDeviceToHost));
+        }
+        GPRAT_CUDA_CHECK(cudaMemcpy(rexp, er.exps.p, rows * sizeof(int32_t), cudaMemcpyDeviceToHost));
+        GPRAT_CUDA_CHECK(
+            cudaMemcpy(bexp, eb.exps.p, ceil_div(rows, 128) * sizeof(int32_t), cudaMemcpyDeviceToHost));
+        set_last_error("");
+        return GPRAT_CU_OK;
+    }
+    catch (const Error &e)
+    {
+        set_last_error(e.what());
+        return e.code;
+    }
+    catch (const std::exception &e)
+    {
+        set_last_error(e.what());
+        return GPRAT_CU_ERR_INVALID_ARG;
+    }
+}
+
 extern "C" int gprat_cu_test_oz_gemm(int M, int N, int K, const double *A, const double *B, double *C, double alpha,
                                      double beta, int lower, int s, int groups, double *rowsq, int max_ctas)
 {

@@ -412,6 +412,29 @@ int gprat_cu_test_oz_gemm(int M,
                           int max_ctas);
 
 /*
+ * Kernel-level test entry (no counterpart in the reference): the product above
+ * with alpha = -1, N even and >= 128, which also writes the digits of the new
+ * C's columns 0 .. 127 from row emit_from (a multiple of 128, < M) on, with
+ * row exponents (rdig, rexp) and block exponents (bdig, bexp): s * rows * 128
+ * bytes, rows and ceil(rows / 128) ints, rows = M - emit_from.  Of these
+ * columns only rows below store_rows are written to C.
+ */
+int gprat_cu_test_oz_emit(int M,
+                          int N,
+                          int K,
+                          const double *A,
+                          const double *B,
+                          double *C,
+                          double beta,
+                          int s,
+                          int emit_from,
+                          int store_rows,
+                          int8_t *rdig,
+                          int32_t *rexp,
+                          int8_t *bdig,
+                          int32_t *bexp);
+
+/*
  * Serving (no counterpart in the reference, whose every predict call
  * re-assembles and re-factorises K, core/src/cpu/gp_functions.cpp:110-189).
  * A server owns fitted models resident on one GPU (factor L and alpha stay

@@ -218,3 +218,37 @@ def test_gemm_each_number_of_groups(capi, G, largest):
     capi.test_oz_gemm(A, B, C, 1.0, 0.0, s, G, False, max_ctas=2)
     ref, mag = np_oz_gemm(A, B, C, 1.0, 0.0, s, G)
     assert np.all(np.abs(C - ref) <= 2.0 ** -46 * mag)
+
+
+@pytest.mark.parametrize("M,N,K,beta,s,emit_from,store_rows", [
+    (512, 128, 128, 0.0, 5, 0, 0),       # digits only
+    (700, 256, 384, 1.0, 5, 128, 128),   # the rows below a diagonal block, several tiles
+    (300, 200, 256, 1.0, 6, 128, 300),   # ragged rows and columns, everything stored
+    (129, 130, 128, 0.0, 3, 128, 129),   # one row
+    (256, 128, 128, 1.0, 7, 0, 77),      # a row range that ends inside a warp's rows
+])
+def test_gemm_writes_the_digits_of_its_result(capi, M, N, K, beta, s, emit_from, store_rows):
+    rng = np.random.default_rng(M + N + s)
+    A, B = graded(rng, M, K), graded(rng, N, K)
+    C = rng.standard_normal((M, N))
+    A[emit_from] = 0.0
+    if beta:
+        C[emit_from] = 0.0            # an all-zero row
+        C[M - 2, 5] = np.nan
+        C[M - 1, 100] = np.inf
+    full = C.copy()
+    rd, re, bd, be = capi.test_oz_emit(A, B, full, beta, s, emit_from, M)
+    plain = C.copy()
+    capi.test_oz_gemm(A, B, plain, -1.0, beta, s)
+    assert np.array_equal(full, plain, equal_nan=True)
+    src = np.ascontiguousarray(full[emit_from:, :128])
+    for block, d, e in ((False, rd, re), (True, bd, be)):
+        ds, es = capi.test_oz_split(src, s, block)
+        assert np.array_equal(e, es)
+        assert np.array_equal(d, ds)
+    part = C.copy()
+    again = capi.test_oz_emit(A, B, part, beta, s, emit_from, store_rows)
+    want = full.copy()
+    want[store_rows:, :128] = C[store_rows:, :128]
+    assert np.array_equal(part, want, equal_nan=True)
+    assert all(np.array_equal(x, y) for x, y in zip(again, (rd, re, bd, be)))
