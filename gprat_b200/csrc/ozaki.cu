@@ -100,14 +100,28 @@ __device__ __forceinline__ int exp_of(double vmax, bool bad)
     return e < -960 ? OZ_ZERO_EXP : e;
 }
 
-// The leading balanced base-254 digit of t, and t <- 254 (t - digit): y holds
-// the digit in its low word, 254 digit is exact from y by one FMA, and the next
-// t is rounded once, as (t - digit) 254 would be (t - digit is exact).
+// The leading balanced base-254 digit of t (the low byte of the result), and
+// t <- 254 (t - digit) if more are wanted: y holds the digit in its low word,
+// 254 digit is exact from y by one FMA, and the next t is rounded once, as
+// (t - digit) 254 would be (t - digit is exact).
+template <bool MORE>
 __device__ __forceinline__ uint32_t next_digit(double &t)
 {
     const double y = __dadd_rn(t, RND);
-    t = __fma_rn(t, OZ_BASE, __fma_rn(y, -OZ_BASE, OZ_BASE * RND));
-    return static_cast<uint32_t>(__double2loint(y)) & 0xffu;
+    if (MORE)
+    {
+        t = __fma_rn(t, OZ_BASE, __fma_rn(y, -OZ_BASE, OZ_BASE * RND));
+    }
+    return static_cast<uint32_t>(__double2loint(y));
+}
+
+// The digits of four consecutive values as bytes.
+template <bool MORE>
+__device__ __forceinline__ uint32_t next_digits(double *t)
+{
+    const uint32_t d0 = next_digit<MORE>(t[0]), d1 = next_digit<MORE>(t[1]);
+    const uint32_t d2 = next_digit<MORE>(t[2]), d3 = next_digit<MORE>(t[3]);
+    return __byte_perm(__byte_perm(d0, d1, 0x0040), __byte_perm(d2, d3, 0x0040), 0x5410);
 }
 
 __device__ __forceinline__ double digit_scale(int e)
@@ -129,13 +143,7 @@ __device__ __forceinline__ void write_digits(const double v[4], int e, int8_t *o
 #pragma unroll
     for (int p = 0; p < S; ++p)
     {
-        uint32_t word = 0;
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-        {
-            word |= next_digit(t[i]) << (8 * i);
-        }
-        *reinterpret_cast<uint32_t *>(out + p * plane) = word;
+        *reinterpret_cast<uint32_t *>(out + p * plane) = p + 1 < S ? next_digits<true>(t) : next_digits<false>(t);
     }
 }
 
@@ -152,16 +160,15 @@ __device__ __forceinline__ void write_row_digits(const double (&v)[64], int e, i
         {
             t[i] = __dmul_rn(v[16 * c + i], sc);
         }
-        for (int p = 0; p < S; ++p)
+        int8_t *dst = out + 16 * c;
+#pragma unroll 1
+        for (int p = 1; p < S; ++p, dst += plane)
         {
-            uint32_t w[4] = { 0, 0, 0, 0 };
-#pragma unroll
-            for (int i = 0; i < 16; ++i)
-            {
-                w[i >> 2] |= next_digit(t[i]) << (8 * (i & 3));
-            }
-            *reinterpret_cast<uint4 *>(out + p * plane + 16 * c) = make_uint4(w[0], w[1], w[2], w[3]);
+            *reinterpret_cast<uint4 *>(dst) = make_uint4(next_digits<true>(t), next_digits<true>(t + 4),
+                                                         next_digits<true>(t + 8), next_digits<true>(t + 12));
         }
+        *reinterpret_cast<uint4 *>(dst) = make_uint4(next_digits<false>(t), next_digits<false>(t + 4),
+                                                     next_digits<false>(t + 8), next_digits<false>(t + 12));
     }
 }
 
@@ -323,6 +330,19 @@ __host__ __device__ constexpr bool oz_sums(int G)
 __host__ __device__ constexpr bool phase_ends(int j, int G)
 {
     return j == G - 1 || (oz_sums(G) ? j == 1 : ((j & 1) != 0) == (G != 7));
+}
+
+// Shared memory by its own address: a generic pointer would order these with
+// the stores to C.
+__device__ __forceinline__ void sts2(uint32_t a, double2 v)
+{
+    asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(a), "d"(v.x), "d"(v.y) : "memory");
+}
+__device__ __forceinline__ double2 lds2(uint32_t a)
+{
+    double2 v;
+    asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(a) : "memory");
+    return v;
 }
 
 // The scout's signal to the MMA issuer: a hardware barrier of their two warps
@@ -1007,8 +1027,15 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
             // with each lane at its own row a tile took 25,000 cycles, most of
             // them waiting for the C values (beta = 1).
             double sq = 0.0;
-            double2 *stage = reinterpret_cast<double2 *>(stages + ew * OZ_STAGE_BYTES);
-            const int cl = lane & 7, rl = lane >> 3;  // this lane moves columns 2 cl, 2 cl + 1 of rows rl + 4 i
+            // opaque, so that the addresses below are formed here and not kept in
+            // registers through the products
+            uint32_t stage = smem_u32(stages + ew * OZ_STAGE_BYTES);
+            int ln = lane;
+            int64_t ldc4 = 4 * p.ldc;
+            asm volatile("" : "+r"(stage), "+r"(ln), "+l"(ldc4));
+            // the 16-byte unit u of row r
+            auto unit = [&](int r, int u) { return stage + static_cast<uint32_t>(r * 128 + ((u ^ (r & 7)) << 4)); };
+            const int cl = ln & 7, rl = ln >> 3;  // this lane moves columns 2 cl, 2 cl + 1 of rows rl + 4 i
             double alpha = p.alpha;
             bool beta = p.beta != 0;
             int mst = p.M;  // rows written
@@ -1023,25 +1050,35 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
                     if (beta)
                     {
                         const double *cptr = p.C + static_cast<int64_t>(row0w + rl) * p.ldc + h * 64 + c * 16 + 2 * cl;
-                        double2 cold[8];
-#pragma unroll
-                        for (int i = 0; i < 8; ++i)
+                        if (row0w + 32 <= p.M)
                         {
-                            cold[i] = row0w + rl + 4 * i < p.M ? *reinterpret_cast<const double2 *>(cptr + 4 * i * p.ldc)
-                                                               : make_double2(0.0, 0.0);
+                            double2 cold[8];
+#pragma unroll
+                            for (int i = 0; i < 8; ++i)
+                            {
+                                cold[i] = *reinterpret_cast<const double2 *>(cptr + i * ldc4);
+                            }
+#pragma unroll
+                            for (int i = 0; i < 8; ++i)
+                            {
+                                const int rr = rl + 4 * i;
+                                sts2(unit(rr, cl), cold[i]);
+                            }
                         }
-#pragma unroll
-                        for (int i = 0; i < 8; ++i)
+                        else
                         {
-                            const int rr = rl + 4 * i;
-                            stage[rr * 8 + (cl ^ (rr & 7))] = cold[i];
+#pragma unroll 1
+                            for (int rr = rl; rr < 32 && row0w + rr < p.M; rr += 4, cptr += ldc4)
+                            {
+                                sts2(unit(rr, cl), *reinterpret_cast<const double2 *>(cptr));
+                            }
                         }
                         __syncwarp();
                     }
 #pragma unroll
                     for (int u = 0; u < 8; ++u)
                     {
-                        const double2 o = beta ? stage[lane * 8 + (u ^ (lane & 7))] : make_double2(0.0, 0.0);
+                        const double2 o = beta ? lds2(unit(ln, u)) : make_double2(0.0, 0.0);
                         double &x = acc[c * 16 + 2 * u], &y = acc[c * 16 + 2 * u + 1];
                         x = __dmul_rn(alpha, x);
                         y = __dmul_rn(alpha, y);
@@ -1056,16 +1093,15 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
                 // the row's maximum (infinity if a value is not finite), shared with
                 // the warp that holds its other half, and the CTA's
                 const bool emits = rvalid && row >= p.emit_from;
-                double m = 0.0;
-                bool nonfinite = false;
+                unsigned long long mb = 0;
 #pragma unroll
                 for (int j = 0; j < 64; ++j)
                 {
-                    const double av = fabs(acc[j]);
-                    nonfinite = nonfinite || !(av <= 1.0e308);
-                    m = fmax(m, av);
+                    mb = max(mb, static_cast<unsigned long long>(__double_as_longlong(acc[j])) & 0x7fffffffffffffffull);
                 }
-                m = !emits ? 0.0 : nonfinite ? __longlong_as_double(0x7ff0000000000000ll) : m;
+                // larger than 1e308 or a NaN: infinity
+                double m = emits ? __longlong_as_double(static_cast<long long>(mb)) : 0.0;
+                m = m <= 1.0e308 ? m : __longlong_as_double(0x7ff0000000000000ll);
                 double *mx = reinterpret_cast<double *>(stages);
                 auto epi_sync = [&]()
                 {
@@ -1152,45 +1188,59 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
                     continue;
                 }
                 const int gc = col0 + 2 * cl;
-                const int gr = row0w + rl;
-                double *cptr = p.C + static_cast<int64_t>(gr) * p.ldc + gc;
+                double *cptr = p.C + static_cast<int64_t>(row0w + rl) * p.ldc + gc;
+                // every element of the chunk is written: no tests (they were most of the time)
+                const bool whole = row0w + 32 <= mst && col0 + 16 <= p.N && (!p.lower || col0 + 15 <= row0w);
                 double2 cold[8];
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
                 {
-                    const int r = gr + 4 * i;
-                    const bool full = r < mst && gc + 1 < p.N && (!p.lower || gc + 1 <= r);
-                    cold[i] = (beta && full) ? *reinterpret_cast<const double2 *>(cptr + 4 * i * p.ldc)
-                                             : make_double2(0.0, 0.0);
+                    cold[i] = whole && beta ? *reinterpret_cast<const double2 *>(cptr + i * ldc4) : make_double2(0.0, 0.0);
                 }
 #pragma unroll
                 for (int u = 0; u < 8; ++u)
                 {
-                    stage[lane * 8 + (u ^ (lane & 7))] =
-                        make_double2(alpha * acc[c * 16 + 2 * u], alpha * acc[c * 16 + 2 * u + 1]);
+                    sts2(unit(ln, u), make_double2(alpha * acc[c * 16 + 2 * u], alpha * acc[c * 16 + 2 * u + 1]));
                 }
                 __syncwarp();
-#pragma unroll
-                for (int i = 0; i < 8; ++i)
+                if (whole)
                 {
-                    const int rr = rl + 4 * i;
-                    const int r = row0w + rr;
-                    double2 o = stage[rr * 8 + (cl ^ (rr & 7))];
-                    const bool ok0 = r < mst && gc < p.N && (!p.lower || gc <= r);
-                    const bool ok1 = r < mst && gc + 1 < p.N && (!p.lower || gc + 1 <= r);
-                    double *dst = cptr + 4 * i * p.ldc;
-                    if (ok0 && ok1)
+#pragma unroll
+                    for (int i0 = 0; i0 < 8; i0 += 4)
                     {
-                        if (beta)
+                        double2 o[4];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
                         {
-                            o.x += cold[i].x;
-                            o.y += cold[i].y;
+                            o[i] = lds2(unit(rl + 4 * (i0 + i), cl));
                         }
-                        *reinterpret_cast<double2 *>(dst) = o;
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                        {
+                            if (beta)
+                            {
+                                o[i].x += cold[i0 + i].x;
+                                o[i].y += cold[i0 + i].y;
+                            }
+                            *reinterpret_cast<double2 *>(cptr + (i0 + i) * ldc4) = o[i];
+                        }
                     }
-                    else if (ok0)
+                }
+                else
+                {
+#pragma unroll 1
+                    for (int rr = rl; rr < 32; rr += 4, cptr += ldc4)
                     {
-                        *dst = beta ? *dst + o.x : o.x;
+                        const int r = row0w + rr;
+                        const double2 o = lds2(unit(rr, cl));
+                        if (r < mst && gc < p.N && (!p.lower || gc <= r))
+                        {
+                            cptr[0] = beta ? cptr[0] + o.x : o.x;
+                            if (gc + 1 < p.N && (!p.lower || gc + 1 <= r))
+                            {
+                                cptr[1] = beta ? cptr[1] + o.y : o.y;
+                            }
+                        }
                     }
                 }
                 __syncwarp();
