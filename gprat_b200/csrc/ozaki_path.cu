@@ -13,9 +13,8 @@
 //
 // Schedule (the same look-ahead as the TF32/BF16 path, reference
 // right_looking_cholesky_tiled, core/src/cpu/tiled_algorithms.cpp:14-57):
-// outer panels of 2048 columns (measured best at n = 32768 among 1024 to
-// 4096, with the whole pipeline timed), inside a panel left-looking over
-// 128-column blocks.  Per block column r0:
+// outer panels of 512 to 2048 columns (oz_panel_blocks), inside a panel
+// left-looking over 128-column blocks.  Per block column r0:
 //   update   K[r0:n, r0:r0+128] -= L[r0:n, K0:r0] L[r0:r0+128, K0:r0]^T, with
 //            the row digits P of the rows below the diagonal block
 //   potrf    L_kk and Linv_k in FP64 (potrf_diag)
@@ -38,12 +37,18 @@ namespace gprat_cu
 namespace
 {
 
-#ifndef GPRAT_OZ_PANEL_BLOCKS
-#define GPRAT_OZ_PANEL_BLOCKS 16  // outer panels of 16 x 128 columns
-#endif
-#ifndef GPRAT_OZ_MAIN_PERCENT
-#define GPRAT_OZ_MAIN_PERCENT 80  // SMs the trailing update holds while the side stream works
-#endif
+// Outer panels of this many 128-column blocks: wide ones so that the trailing
+// updates read the digits of C's rows and columns fewer times, narrow ones where
+// the panel chain, whose in-panel updates are left-looking and of 128 columns,
+// isn't hidden by them.  ms per predict_with_uncertainty with 4 / 8 / 16 blocks:
+// n = 4096 4.29 / 4.57 / 5.11, 8192 8.37 / 8.68 / 10.0, 12288 18.6 / 18.6 / 20.8,
+// 16384 - / 31.6 / 33.4, 24576 87.4 / 80.7 / 79.0, 32768 - / 215 / 205.
+int oz_panel_blocks(int n) { return knob("GPRAT_CU_OZ_PANEL_BLOCKS", n <= 8192 ? 4 : n <= 20480 ? 8 : 16, 1, 64); }
+
+// The SMs that the trailing update holds while the side stream factors the
+// next panel, in percent: as many as leave the panel chain hidden.  80 / 86 /
+// 92 %: n = 16384 31.6 / 31.9 / 32.4 ms, 32768 204.8 / 202.4 / 202.8.
+int oz_main_percent(int n) { return sm_percent("GPRAT_CU_OZ_MAIN_PERCENT", n <= 20480 ? 80 : 86); }
 
 // Digit-plane operands of one handle (TMA maps built per call: cheap host work).
 struct OzOps
@@ -131,14 +136,14 @@ void factor_oz(gprat_cu_gp *gp, cudaStream_t s, const std::vector<std::pair<int,
     }
     const int64_t ld = gp->ld;
     const OzOps ops = make_oz_ops(gp);
-    const int nbo = NB * knob("GPRAT_CU_OZ_PANEL_BLOCKS", GPRAT_OZ_PANEL_BLOCKS, 1, 64);
+    const int nbo = NB * oz_panel_blocks(n);
     const int nout = ceil_div(n, nbo);
     ensure_lookahead(gp, lookahead_events(n));
     cudaStream_t side = gp->side;
     auto evF = [&](int k) { return gp->events[1 + k]; };
     auto evR = [&](int k) { return gp->events[1 + nout + k]; };
     const int sms = device_sm_count();
-    const int main_ctas = std::max(2, sms * sm_percent("GPRAT_CU_OZ_MAIN_PERCENT", GPRAT_OZ_MAIN_PERCENT) / 100);
+    const int main_ctas = std::max(2, sms * oz_main_percent(n) / 100);
     // digit groups of the trailing updates (0 = every group); the panel chain
     // (in-panel updates, panel solves) always keeps every group: the factor's
     // accuracy near the diagonal sets alpha's
