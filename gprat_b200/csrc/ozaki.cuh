@@ -83,7 +83,7 @@ struct OzGemmArgs
     DeviceStatus *status;  // timeout flag if a bounded wait gives up
     int max_ctas;          // persistent grid bound (0 = every SM), leaves SMs to other streams
     int groups;            // digit groups kept, 1..s (0 = s)
-    // optional (not lower, N >= 128): the digits of C's new first 128 columns,
+    // optional (not lower, N >= 128, alpha 1 or -1): the digits of C's new first 128 columns,
     // rows [emit_from, M), as rows of emit_row and / or emit_blk (same s as A)
     // from emit_row0 + emit_from on and columns from emit_col0 on: what
     // oz_split would write from C.  emit_col0 a multiple of 128; for emit_blk,
