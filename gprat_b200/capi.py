@@ -347,7 +347,7 @@ class CudaGP:
         out = np.empty(nt * nt * t * t)
         check(lib.gprat_cu_cholesky(self._h, _p(_hyper(hyper)), _p(out)))
         tiles = out.reshape(nt * nt, t * t)
-        return [tiles[i * nt + j].copy() if j <= i else None for i in range(nt) for j in range(nt)]
+        return [tiles[i * nt + j] if j <= i else None for i in range(nt) for j in range(nt)]
 
     def predict(self, hyper, xt, m_tiles: int, m_tile_size: int) -> np.ndarray:
         xt = _arr(xt)

@@ -365,7 +365,29 @@ __global__ void __launch_bounds__(32 * MV_WARPS) cross_mv_kernel(const double *_
         mean[r] = s;
     }
 }
+
+// One block per line: line l of a tile row holds row l % T of its tile l / T.
+__global__ void __launch_bounds__(256) pack_lines_kernel(const double *__restrict__ K, int64_t ld, int T, int64_t l0,
+                                                         double *__restrict__ out)
+{
+    const int64_t l = l0 + blockIdx.x;
+    const double *src = K + (l % T) * ld + l / T * T;
+    double *dst = out + static_cast<int64_t>(blockIdx.x) * T;
+    for (int c = threadIdx.x; c < T; c += 256)
+    {
+        dst[c] = src[c];
+    }
+}
 }  // namespace
+
+void pack_lines(const double *K, int64_t ld, int T, int64_t l0, int lines, double *out, cudaStream_t s)
+{
+    if (lines > 0)
+    {
+        pack_lines_kernel<<<lines, 256, 0, s>>>(K, ld, T, l0, out);
+        GPRAT_LAUNCH_CHECK();
+    }
+}
 
 void cross_times_alpha(const double *Kx, int64_t ldx, int m, int n, const double *alpha, double *mean, cudaStream_t s,
                        bool upper)

@@ -223,6 +223,10 @@ void assemble_cross_dual(const double *xt, int m, const double *x, int n, int n_
 // is zero left of column r (not read).
 void cross_times_alpha(const double *Kx, int64_t ldx, int m, int n, const double *alpha, double *mean, cudaStream_t s,
                        bool upper = false);
+// out := lines l0 .. l0 + lines - 1 of a tile row of the matrix whose first row is
+// K, T values each: its T x T tiles from the left, row by row.
+void pack_lines(const double *K, int64_t ld, int T, int64_t l0, int lines, double *out, cudaStream_t s);
+
 void reduce_mean(const double *mean_partial, int m, int parts, double *mean, cudaStream_t s);
 
 // Prior covariance matrix K**[r][c] = k(xt_r, xt_c) (gen_tile_full_prior_covariance,

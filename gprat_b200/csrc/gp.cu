@@ -903,29 +903,29 @@ int gprat_cu_cholesky(gprat_cu_gp *gp, const double hyper[3], double *tiles_out)
             SolveRows none{};
             none.c_first = true;
             factor_fp64(gp, none, gp->stream);
-            std::vector<double> full(static_cast<size_t>(gp->n) * gp->ld);
-            download(gp, full.data(), gp->K.ptr, static_cast<int64_t>(gp->n) * gp->ld);
             finish_and_check(gp);
+            // The tiles are put in order on the device, a part of a tile row at a
+            // time, and copied straight to where they belong: copying the whole
+            // matrix into a host buffer of its own and from there tile by tile
+            // took twenty times as long as the factorisation at n = 2048.
+            constexpr int64_t PART = int64_t(1) << 23;  // 64 MB
             const int T = gp->T, nt = gp->n_tiles;
             const size_t tt = static_cast<size_t>(T) * T;
+            const int part = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(PART / T, int64_t(nt) * T)));
+            gp->W.ensure(static_cast<int64_t>(part) * T);
             for (int i = 0; i < nt; ++i)
             {
-                for (int j = 0; j < nt; ++j)
+                double *row = tiles_out + static_cast<size_t>(i) * nt * tt;
+                const int64_t lines = static_cast<int64_t>(i + 1) * T;
+                for (int64_t l = 0; l < lines; l += part)
                 {
-                    double *dst = tiles_out + (static_cast<size_t>(i) * nt + j) * tt;
-                    if (j > i)
-                    {
-                        std::memset(dst, 0, tt * sizeof(double));
-                        continue;
-                    }
-                    for (int r = 0; r < T; ++r)
-                    {
-                        std::memcpy(dst + static_cast<size_t>(r) * T,
-                                    full.data() + static_cast<size_t>(i * T + r) * gp->ld + static_cast<size_t>(j) * T,
-                                    T * sizeof(double));
-                    }
+                    const int count = static_cast<int>(std::min<int64_t>(part, lines - l));
+                    pack_lines(gp->K.ptr + static_cast<int64_t>(i) * T * gp->ld, gp->ld, T, l, count, gp->W.ptr, gp->stream);
+                    download(gp, row + l * T, gp->W.ptr, static_cast<int64_t>(count) * T);
                 }
+                std::memset(row + static_cast<size_t>(i + 1) * tt, 0, static_cast<size_t>(nt - i - 1) * tt * sizeof(double));
             }
+            GPRAT_CUDA_CHECK(cudaStreamSynchronize(gp->stream));
         });
 }
 
