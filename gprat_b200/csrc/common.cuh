@@ -261,14 +261,17 @@ void trsv_fused_forward(const double *L, int64_t ld, const double *Linv, int n, 
                         double *scratch, DeviceStatus *st, cudaStream_t s, int max_ctas = 0);
 void trsv_fused_backward(const double *L, int64_t ld, const double *Linv, int n, double *x, int *flags,
                          double *scratch, DeviceStatus *st, cudaStream_t s, int max_ctas = 0);
-// skip (optional, device): when *skip != 0 at launch the solve returns at once
-// (a preconditioner step of an already converged CG iteration)
 void trsv_fused_forward_f32(const float *L, int64_t ld, const float *Linv, int n, double *x, int *flags,
-                            double *scratch, DeviceStatus *st, cudaStream_t s, int max_ctas = 0,
-                            const int *skip = nullptr);
+                            double *scratch, DeviceStatus *st, cudaStream_t s, int max_ctas = 0);
 void trsv_fused_backward_f32(const float *L, int64_t ld, const float *Linv, int n, double *x, int *flags,
-                             double *scratch, DeviceStatus *st, cudaStream_t s, int max_ctas = 0,
-                             const int *skip = nullptr);
+                             double *scratch, DeviceStatus *st, cudaStream_t s, int max_ctas = 0);
+// The same from b into x, whose bytes the caller has set to 0xFF and *ticket to
+// 0.  skip (optional, device): when *skip != 0 at launch the solve returns at
+// once (a preconditioner step of an already converged CG iteration).
+void trsv_forward_f32(const float *L, int64_t ld, const float *Linv, int n, const double *b, double *x, int *ticket,
+                      DeviceStatus *st, cudaStream_t s, int max_ctas, const int *skip);
+void trsv_backward_f32(const float *L, int64_t ld, const float *Linv, int n, const double *b, double *x, int *ticket,
+                       DeviceStatus *st, cudaStream_t s, int max_ctas, const int *skip);
 // Poll budget of the bounded waits on the current device: the single-launch
 // solves' on an unsolved block and the FP64 products' on their operand copies
 // (polls < 0: the defaults, about 0.5-1 s and 2 s).

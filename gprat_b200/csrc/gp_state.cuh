@@ -78,6 +78,7 @@ struct PcgScalars
     double a, b;    // step lengths
     int converged;  // 1 once |r| <= tol |y|
     int iters;      // iterations taken
+    unsigned arrived;  // CTAs of the running dot product that have stored their part
 };
 
 }  // namespace gprat_cu

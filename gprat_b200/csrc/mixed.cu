@@ -265,42 +265,27 @@ __global__ void __launch_bounds__(SV_THREADS) symv_tile_kernel(const double *__r
     }
 }
 
-__global__ void symv_reduce_kernel(const double *__restrict__ part, int nblk, int n, double *__restrict__ q,
-                                   const int *skip)
-{
-    if (*skip != 0)
-    {
-        return;
-    }
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n)
-    {
-        double s = 0.0;
-        for (int b = 0; b < nblk; ++b)
-        {
-            s += part[static_cast<int64_t>(b) * n + i];
-        }
-        q[i] = s;
-    }
-}
-
 // ---------------------------------------------------------------------------
-// PCG helpers (all scalars live in PcgScalars on the device)
+// PCG helpers (all scalars live in PcgScalars on the device).
+//
+// An iteration is seven launches: the product's tiles, its sums with p . q, the
+// update with r . r, the two solves, r . z and the new direction.  Every dot
+// product rides along with what produces its vector, the last CTA to finish
+// forms the scalar that follows from it, and the solves' outputs and tickets are
+// reset by the update; as kernels, copies and fills of their own these were
+// seventeen, 1.2 to 2 us each, on a chain of 24 iterations (n = 4096: 1.2 of
+// 2.6 ms; launches after convergence return at once but are still made).
 
-__global__ void __launch_bounds__(DOT_THREADS) dot_partial_kernel(const double *__restrict__ a,
-                                                                  const double *__restrict__ b, int n,
-                                                                  double *__restrict__ part, const int *skip)
+// The CTAs that a dot product of n values takes; the sum's order is that of
+// DOT_BLOCKS parts, of which the others are zero.
+int dot_blocks(int n) { return std::min(DOT_BLOCKS, ceil_div(n, DOT_THREADS)); }
+
+// Adds the CTA's values s to part[] and, in the last CTA, sums the parts in order
+// and sets what depends on the product.
+// which: 0 = yy (init), 1 = rz (init), 2 = pq -> a, 3 = rr -> converged, 4 = rz -> b
+__device__ void finish_dot(double s, double *part, PcgScalars *ps, int which, double tol)
 {
-    if (skip != nullptr && *skip != 0)
-    {
-        return;
-    }
     __shared__ double red[DOT_THREADS];
-    double s = 0.0;
-    for (int i = blockIdx.x * DOT_THREADS + threadIdx.x; i < n; i += DOT_BLOCKS * DOT_THREADS)
-    {
-        s += a[i] * b[i];
-    }
     red[threadIdx.x] = s;
     __syncthreads();
     for (int w = DOT_THREADS / 2; w > 0; w >>= 1)
@@ -311,73 +296,140 @@ __global__ void __launch_bounds__(DOT_THREADS) dot_partial_kernel(const double *
         }
         __syncthreads();
     }
-    if (threadIdx.x == 0)
-    {
-        part[blockIdx.x] = red[0];
-    }
-}
-
-__device__ double sum_parts(const double *part)
-{
-    double s = 0.0;
-    for (int b = 0; b < DOT_BLOCKS; ++b)
-    {
-        s += part[b];
-    }
-    return s;
-}
-
-// which: 0 = yy (init), 1 = rz (init), 2 = pq -> a, 3 = rr -> converged, 4 = rz -> b
-__global__ void pcg_scalar_kernel(PcgScalars *s, const double *part, int which, double tol)
-{
-    if (threadIdx.x != 0 || blockIdx.x != 0)
+    if (threadIdx.x != 0)
     {
         return;
     }
-    if (which >= 2 && s->converged != 0)
+    part[blockIdx.x] = red[0];
+    __threadfence();
+    if (atomicAdd(&ps->arrived, 1u) != gridDim.x - 1)
     {
-        return;  // an iteration after convergence: nothing changes
+        return;
     }
-    const double v = sum_parts(part);
+    __threadfence();
+    ps->arrived = 0;
+    double v = 0.0;
+    for (unsigned b = 0; b < gridDim.x; ++b)
+    {
+        v += __ldcg(part + b);
+    }
     switch (which)
     {
         case 0:
-            s->yy = v;
-            s->converged = (v == 0.0) ? 1 : 0;
-            s->iters = 0;
+            ps->yy = v;
+            ps->converged = (v == 0.0) ? 1 : 0;
+            ps->iters = 0;
             break;
-        case 1: s->rz = v; break;
+        case 1: ps->rz = v; break;
         case 2:
-            s->pq = v;
-            s->a = (v != 0.0) ? s->rz / v : 0.0;
+            ps->pq = v;
+            ps->a = (v != 0.0) ? ps->rz / v : 0.0;
             break;
         case 3:
-            s->rr = v;
-            s->iters += 1;
-            s->converged = (v <= tol * tol * s->yy) ? 1 : 0;
+            ps->rr = v;
+            ps->iters += 1;
+            ps->converged = (v <= tol * tol * ps->yy) ? 1 : 0;
             break;
         case 4:
-            s->b = (s->rz != 0.0) ? v / s->rz : 0.0;
-            s->rz = v;
+            ps->b = (ps->rz != 0.0) ? v / ps->rz : 0.0;
+            ps->rz = v;
             break;
     }
 }
 
-// x += a p; r -= a q
-__global__ void pcg_update_kernel(const PcgScalars *__restrict__ s, double *__restrict__ x,
-                                  double *__restrict__ r, const double *__restrict__ p,
-                                  const double *__restrict__ q, int n)
+// What a solve waits for is marked by the bytes 0xFF (trsv_fused.cu).
+__device__ double unsolved() { return __longlong_as_double(-1ll); }
+
+// x = 0, r = y, y . y; the solves' outputs zf, z and tickets reset
+__global__ void __launch_bounds__(DOT_THREADS) pcg_init_kernel(const double *__restrict__ y, double *__restrict__ x,
+                                                               double *__restrict__ r, double *__restrict__ zf,
+                                                               double *__restrict__ z, int *tickets, int n,
+                                                               double *part, PcgScalars *ps)
 {
-    if (s->converged != 0)
+    double s = 0.0;
+    for (int i = blockIdx.x * DOT_THREADS + threadIdx.x; i < n; i += DOT_BLOCKS * DOT_THREADS)
+    {
+        const double v = y[i];
+        x[i] = 0.0;
+        r[i] = v;
+        zf[i] = unsolved();
+        z[i] = unsolved();
+        s += v * v;
+    }
+    if (blockIdx.x == 0 && threadIdx.x < 2)
+    {
+        tickets[threadIdx.x] = 0;
+    }
+    finish_dot(s, part, ps, 0, 0.0);
+}
+
+// q = the sum of the tiles' parts, p . q
+__global__ void __launch_bounds__(DOT_THREADS) symv_reduce_kernel(const double *__restrict__ tiles, int nblk, int n,
+                                                                  const double *__restrict__ p, double *__restrict__ q,
+                                                                  double *part, PcgScalars *ps)
+{
+    if (ps->converged != 0)
     {
         return;
     }
-    const double a = s->a;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    double s = 0.0;
+    for (int i = blockIdx.x * DOT_THREADS + threadIdx.x; i < n; i += DOT_BLOCKS * DOT_THREADS)
+    {
+        double v = 0.0;
+        for (int b = 0; b < nblk; ++b)
+        {
+            v += tiles[static_cast<int64_t>(b) * n + i];
+        }
+        q[i] = v;
+        s += p[i] * v;
+    }
+    finish_dot(s, part, ps, 2, 0.0);
+}
+
+// x += a p; r -= a q; r . r; the solves' outputs and tickets reset
+__global__ void __launch_bounds__(DOT_THREADS) pcg_update_kernel(double *__restrict__ x, double *__restrict__ r,
+                                                                 const double *__restrict__ p,
+                                                                 const double *__restrict__ q, double *__restrict__ zf,
+                                                                 double *__restrict__ z, int *tickets, int n,
+                                                                 double *part, PcgScalars *ps, double tol)
+{
+    if (ps->converged != 0)
+    {
+        return;
+    }
+    const double a = ps->a;
+    double s = 0.0;
+    for (int i = blockIdx.x * DOT_THREADS + threadIdx.x; i < n; i += DOT_BLOCKS * DOT_THREADS)
     {
         x[i] += a * p[i];
-        r[i] -= a * q[i];
+        const double v = r[i] - a * q[i];
+        r[i] = v;
+        zf[i] = unsolved();
+        z[i] = unsolved();
+        s += v * v;
     }
+    if (blockIdx.x == 0 && threadIdx.x < 2)
+    {
+        tickets[threadIdx.x] = 0;
+    }
+    finish_dot(s, part, ps, 3, tol);
+}
+
+// r . z
+__global__ void __launch_bounds__(DOT_THREADS) pcg_dot_kernel(const double *__restrict__ r,
+                                                              const double *__restrict__ z, int n, double *part,
+                                                              PcgScalars *ps, int which)
+{
+    if (ps->converged != 0)
+    {
+        return;
+    }
+    double s = 0.0;
+    for (int i = blockIdx.x * DOT_THREADS + threadIdx.x; i < n; i += DOT_BLOCKS * DOT_THREADS)
+    {
+        s += r[i] * z[i];
+    }
+    finish_dot(s, part, ps, which, 0.0);
 }
 
 // p = z + b p
@@ -395,41 +447,17 @@ __global__ void pcg_direction_kernel(const PcgScalars *__restrict__ s, double *_
     }
 }
 
-// skip (optional, device): the product is not needed when *skip != 0
-void dot(const double *a, const double *b, int n, double *part, cudaStream_t s, const int *skip = nullptr)
-{
-    dot_partial_kernel<<<DOT_BLOCKS, DOT_THREADS, 0, s>>>(a, b, n, part, skip);
-    GPRAT_LAUNCH_CHECK();
-}
-
-void scalar(PcgScalars *ps, const double *part, int which, cudaStream_t s)
-{
-    pcg_scalar_kernel<<<1, 32, 0, s>>>(ps, part, which, pcg_tol());
-    GPRAT_LAUNCH_CHECK();
-}
-
 int blocks_for(int n) { return std::min(ceil_div(n, 256), 148 * 8); }
 
-void symv(gprat_cu_gp *gp, const double *p, double *q, cudaStream_t s, const int *skip)
-{
-    const int tiles = gp->nblk * (gp->nblk + 1) / 2;
-    symv_tile_kernel<<<tiles, SV_THREADS, 0, s>>>(gp->K.ptr, gp->ld, gp->n, p, gp->symv_part.ptr, skip);
-    GPRAT_LAUNCH_CHECK();
-    symv_reduce_kernel<<<ceil_div(gp->n, 256), 256, 0, s>>>(gp->symv_part.ptr, gp->nblk, gp->n, q, skip);
-    GPRAT_LAUNCH_CHECK();
-}
-
-// z = (L L^T)^-1 r with the low-precision factor; solve_ctas > 0 bounds the
-// solves' grids; nothing is solved when *skip != 0.
+// z = (L L^T)^-1 r with the low-precision factor (outputs and tickets reset
+// before); solve_ctas > 0 bounds the solves' grids; nothing is solved when
+// *skip != 0.
 void precondition(gprat_cu_gp *gp, const double *r, double *z, cudaStream_t s, int solve_ctas, const int *skip)
 {
-    GPRAT_CUDA_CHECK(cudaMemcpyAsync(z, r, gp->n * sizeof(double), cudaMemcpyDeviceToDevice, s));
-    gp->flags.ensure(2);
-    gp->trsv_b.ensure(gp->n);
-    trsv_fused_forward_f32(gp->K32.ptr, gp->ld32, gp->Linv32.ptr, gp->n, z, gp->flags.ptr, gp->trsv_b.ptr,
-                           gp->status.ptr, s, solve_ctas, skip);
-    trsv_fused_backward_f32(gp->K32.ptr, gp->ld32, gp->Linv32.ptr, gp->n, z, gp->flags.ptr, gp->trsv_b.ptr,
-                            gp->status.ptr, s, solve_ctas, skip);
+    trsv_forward_f32(gp->K32.ptr, gp->ld32, gp->Linv32.ptr, gp->n, r, gp->trsv_b.ptr, gp->flags.ptr, gp->status.ptr, s,
+                     solve_ctas, skip);
+    trsv_backward_f32(gp->K32.ptr, gp->ld32, gp->Linv32.ptr, gp->n, gp->trsv_b.ptr, z, gp->flags.ptr + 1,
+                      gp->status.ptr, s, solve_ctas, skip);
 }
 
 }  // namespace
@@ -678,32 +706,35 @@ void alpha_mixed(gprat_cu_gp *gp, cudaStream_t s, int solve_ctas)
     }
     gp->symv_part.ensure(static_cast<int64_t>(gp->nblk) * n + 3 * DOT_BLOCKS);
     gp->pcg_s.ensure(1);
+    gp->flags.ensure(2);
+    gp->trsv_b.ensure(n);
     double *part = gp->symv_part.ptr + static_cast<int64_t>(gp->nblk) * n;  // dot partials
     PcgScalars *ps = gp->pcg_s.ptr;
     double *x = gp->alpha.ptr, *r = gp->pcg_r.ptr, *z = gp->pcg_z.ptr, *p = gp->pcg_p.ptr, *q = gp->pcg_q.ptr;
-    const int nb = blocks_for(n);
+    double *zf = gp->trsv_b.ptr;
+    int *tickets = gp->flags.ptr;
+    const int nb = blocks_for(n), db = dot_blocks(n), tiles = gp->nblk * (gp->nblk + 1) / 2;
+    const double tol = pcg_tol();
 
     const int *done = &ps->converged;  // device flag, set by the residual test
-    GPRAT_CUDA_CHECK(cudaMemsetAsync(x, 0, n * sizeof(double), s));
-    GPRAT_CUDA_CHECK(cudaMemcpyAsync(r, gp->y.ptr, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
-    dot(r, r, n, part, s);
-    scalar(ps, part, 0, s);
+    GPRAT_CUDA_CHECK(cudaMemsetAsync(ps, 0, sizeof(PcgScalars), s));
+    pcg_init_kernel<<<db, DOT_THREADS, 0, s>>>(gp->y.ptr, x, r, zf, z, tickets, n, part, ps);
+    GPRAT_LAUNCH_CHECK();
     precondition(gp, r, z, s, solve_ctas, done);
-    dot(r, z, n, part, s, done);
-    scalar(ps, part, 1, s);
+    pcg_dot_kernel<<<db, DOT_THREADS, 0, s>>>(r, z, n, part, ps, 1);
+    GPRAT_LAUNCH_CHECK();
     GPRAT_CUDA_CHECK(cudaMemcpyAsync(p, z, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
     for (int it = 0; it < PCG_ITERS; ++it)
     {
-        symv(gp, p, q, s, done);
-        dot(p, q, n, part, s, done);
-        scalar(ps, part, 2, s);
-        pcg_update_kernel<<<nb, 256, 0, s>>>(ps, x, r, p, q, n);
+        symv_tile_kernel<<<tiles, SV_THREADS, 0, s>>>(gp->K.ptr, gp->ld, n, p, gp->symv_part.ptr, done);
         GPRAT_LAUNCH_CHECK();
-        dot(r, r, n, part, s, done);
-        scalar(ps, part, 3, s);
+        symv_reduce_kernel<<<db, DOT_THREADS, 0, s>>>(gp->symv_part.ptr, gp->nblk, n, p, q, part, ps);
+        GPRAT_LAUNCH_CHECK();
+        pcg_update_kernel<<<db, DOT_THREADS, 0, s>>>(x, r, p, q, zf, z, tickets, n, part, ps, tol);
+        GPRAT_LAUNCH_CHECK();
         precondition(gp, r, z, s, solve_ctas, done);
-        dot(r, z, n, part, s, done);
-        scalar(ps, part, 4, s);
+        pcg_dot_kernel<<<db, DOT_THREADS, 0, s>>>(r, z, n, part, ps, 4);
+        GPRAT_LAUNCH_CHECK();
         pcg_direction_kernel<<<nb, 256, 0, s>>>(ps, p, z, n);
         GPRAT_LAUNCH_CHECK();
     }

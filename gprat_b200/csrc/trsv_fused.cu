@@ -939,34 +939,44 @@ void trsv_fused_backward(const double *L, int64_t ld, const double *Linv, int n,
     bwd(L, ld, Linv, n, x, flags, scratch, st, s, max_ctas);
 }
 
-void trsv_fused_forward_f32(const float *L, int64_t ld, const float *Linv, int n, double *x, int *flags,
-                            double *scratch, DeviceStatus *st, cudaStream_t s, int max_ctas, const int *skip)
+void trsv_forward_f32(const float *L, int64_t ld, const float *Linv, int n, const double *b, double *x, int *ticket,
+                      DeviceStatus *st, cudaStream_t s, int max_ctas, const int *skip)
 {
     if ((ld & 3) != 0 || (reinterpret_cast<uintptr_t>(L) & 15) != 0 || (reinterpret_cast<uintptr_t>(Linv) & 15) != 0)
     {
-        throw Error(1, "trsv_fused_forward_f32: L and Linv must be 16-byte aligned, ld a multiple of 4");
+        throw Error(1, "trsv_forward_f32: L and Linv must be 16-byte aligned, ld a multiple of 4");
     }
-    const int nblk = ceil_div(n, FB);
     ensure_smem_attr(reinterpret_cast<const void *>(trsv_fwd_f32_kernel), static_cast<int>(SMEM_F32_FWD));
-    prepare(x, scratch, n, flags, s);
-    trsv_fwd_f32_kernel<<<grid_for(nblk, max_ctas), FT, SMEM_F32_FWD, s>>>(L, ld, Linv, n, scratch, x, flags, st,
-                                                                        skip);
+    trsv_fwd_f32_kernel<<<grid_for(ceil_div(n, FB), max_ctas), FT, SMEM_F32_FWD, s>>>(L, ld, Linv, n, b, x, ticket, st,
+                                                                                   skip);
     GPRAT_LAUNCH_CHECK();
 }
 
-void trsv_fused_backward_f32(const float *L, int64_t ld, const float *Linv, int n, double *x, int *flags,
-                             double *scratch, DeviceStatus *st, cudaStream_t s, int max_ctas, const int *skip)
+void trsv_backward_f32(const float *L, int64_t ld, const float *Linv, int n, const double *b, double *x, int *ticket,
+                       DeviceStatus *st, cudaStream_t s, int max_ctas, const int *skip)
 {
     if ((ld & 3) != 0 || (reinterpret_cast<uintptr_t>(L) & 15) != 0 || (reinterpret_cast<uintptr_t>(Linv) & 15) != 0)
     {
-        throw Error(1, "trsv_fused_backward_f32: L and Linv must be 16-byte aligned, ld a multiple of 4");
+        throw Error(1, "trsv_backward_f32: L and Linv must be 16-byte aligned, ld a multiple of 4");
     }
     const int nblk = ceil_div(n, FB);
     ensure_smem_attr(reinterpret_cast<const void *>(trsv_bwd_f32_kernel), static_cast<int>(SMEM_F32_BWD));
-    prepare(x, scratch, n, flags, s);
-    trsv_bwd_f32_kernel<<<grid_for(nblk, max_ctas), FT, SMEM_F32_BWD, s>>>(L, ld, Linv, n, nblk, scratch, x, flags,
-                                                                        st, skip);
+    trsv_bwd_f32_kernel<<<grid_for(nblk, max_ctas), FT, SMEM_F32_BWD, s>>>(L, ld, Linv, n, nblk, b, x, ticket, st, skip);
     GPRAT_LAUNCH_CHECK();
+}
+
+void trsv_fused_forward_f32(const float *L, int64_t ld, const float *Linv, int n, double *x, int *flags,
+                            double *scratch, DeviceStatus *st, cudaStream_t s, int max_ctas)
+{
+    prepare(x, scratch, n, flags, s);
+    trsv_forward_f32(L, ld, Linv, n, scratch, x, flags, st, s, max_ctas, nullptr);
+}
+
+void trsv_fused_backward_f32(const float *L, int64_t ld, const float *Linv, int n, double *x, int *flags,
+                             double *scratch, DeviceStatus *st, cudaStream_t s, int max_ctas)
+{
+    prepare(x, scratch, n, flags, s);
+    trsv_backward_f32(L, ld, Linv, n, scratch, x, flags, st, s, max_ctas, nullptr);
 }
 
 // Sets the poll budget of the solves' waits on the current device; polls < 0
