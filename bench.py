@@ -254,6 +254,13 @@ def measure_int8_peak(torch, device) -> float:
     return best
 
 
+def reference_missing():
+    """Why the compiled reference cannot be timed here, or None."""
+    from oracle import ref
+
+    return None if ref.available() else "the compiled reference (oracle/_ref) is not built here"
+
+
 def cpu_reference_full(wl, reps: int):
     """The reference's own CPU path (compiled from source, oracle/_ref) at the
     FULL workload on all host cores: `reps` timed predict_with_uncertainty
@@ -435,6 +442,10 @@ REF_FULL_REPS = 2
 def run_reference(args, wl):
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
+        return
+    missing = reference_missing()
+    if missing:
+        print(json.dumps({"impl": "reference", "unavailable": missing}), flush=True)
         return
     reps = min(max(args.steps, 1), REF_FULL_REPS)
     times, desc, threads = cpu_reference_full(wl, reps)
@@ -784,7 +795,14 @@ def run_ours(args, wl):
     if gemm_tflops and "tf32_half_rate" in extra_peaks:
         extra_peaks["frac_of_tf32_half_rate"] = gemm_tflops / extra_peaks["tf32_half_rate"]
     step_flops = algorithmic_flops(n, m)
-    if world == 1 and not args.skip_cpu_baseline:
+    missing = reference_missing()
+    if world == 1 and not args.skip_cpu_baseline and missing:
+        cpu = {"unavailable": missing,
+               "gpu_calls_at_sample": {"fp64": gpu_calls(wl, capi.PREC_FP64),
+                                       args.precision: gpu_calls(wl, args.precision)}}
+        if not args.skip_c3:
+            cpu["c3_optimize"] = c3_optimize(reference=False)
+    elif world == 1 and not args.skip_cpu_baseline:
         times, desc, threads = cpu_reference_full(wl, 1)
         cpu = {"value": times[0], "unit": "s", "cores": threads, "kind": "reference", "sample": desc,
                "calls_at_sample": cpu_reference_calls(wl),
