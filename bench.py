@@ -762,7 +762,7 @@ def run_ours(args, wl):
     extra_peaks = {}
     if args.precision == "fp64":
         peak = measure_fp64_gemm_peak(torch, device)
-        kernel = "dgemm_kernel (FP64 DMMA m16n8k8: Cholesky panel/trailing updates + variance solve)"
+        kernel = "update_kernel, solve_kernel (FP64 DMMA m16n8k8: Cholesky panel/trailing updates + variance solve)"
         peak_source = ("cuBLAS DGEMM (torch.matmul fp64 8192^3, best of 5) measured in this run; "
                        "MEASURED_PEAKS.json holds no FP64 figure")
     elif args.precision.startswith("fp64-int8"):
