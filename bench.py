@@ -498,9 +498,9 @@ TRAFFIC_SAMPLE = {
     "fp64-int8": {
         "launch": "oz_gemm_kernel, every launch of one fit+predict step at n_train=32768, 5 digit planes "
                   "(1035 launches, 1-pass ncu launch list); per-launch mean below; largest launch (variance top "
-                  "update 8192 x 16384 x 16384): 35.86 GB DRAM against 4.1 GB algorithmic",
-        "dram_bytes": 208.86e9 / 1035,
-        "dram_bytes_step": 208.86e9,
+                  "update 8192 x 16384 x 16384): 73.98 GB DRAM against 4.1 GB algorithmic",
+        "dram_bytes": 282.19e9 / 1035,
+        "dram_bytes_step": 282.19e9,
         "workload": "c2",
         "source": "profiles/launch_list_fit_predict_c2_fp64_int8.md",
     },
@@ -512,10 +512,10 @@ TRAFFIC_SAMPLE = {
         "source": "profiles/tc_gemm_trailing_update_c1.md",
     },
     "fp64": {
-        "launch": "dgemm_kernel<2,0,1>, trailing update after the first outer panel at n_train=16384: "
-                  "lower 15872 x 15872, K=512",
-        "dram_bytes": 2.524e9 + 0.986e9,
-        "algorithmic_bytes": 2 * 15872 * 15873 / 2 * 8 + 15872 * 512 * 8,
+        "launch": "update_kernel<2,4,3,false>, trailing update after the first outer panel at n_train=16384: "
+                  "lower 15360 x 15360 and 4096 x 15360 test rows, K=512",
+        "dram_bytes": 3.842e9 + 1.430e9,
+        "algorithmic_bytes": 2 * (15360 * 15361 / 2 + 4096 * 15360) * 8 + (16384 - 512 + 4096) * 512 * 8,
         "source": "profiles/dgemm_trailing_update_c1.md",
     },
 }
