@@ -4,8 +4,8 @@
 // rows are sliding windows of one series (compute_covariance_function,
 // core/src/cpu/gp_algorithms.cpp:11-28; GPU twin core/src/gpu/gp_algorithms.cu:16-55).
 //
-// One CTA produces a 64-row x 128-column block.  The two windows of the
-// series it needs (64+d-1 and 128+d-1 values) are staged in shared memory
+// One CTA produces a block of 64 rows (16 of a small matrix) x 128 columns.  The
+// two windows of the series it needs (64+d-1 and 128+d-1 values) are staged in shared memory
 // once; each thread owns one column and walks the rows, so row values are
 // shared-memory broadcasts and column values are conflict-free.  Every row of
 // the block is written by whole warps as contiguous 256-byte segments
@@ -28,7 +28,6 @@ namespace gprat_cu
 namespace
 {
 
-constexpr int AR = 64;   // rows per CTA
 constexpr int AC = 128;  // columns per CTA (= threads)
 constexpr int RB = 4;    // rows per inner pass
 
@@ -77,7 +76,8 @@ constexpr int RECUR_MIN_D = 16;
 // mode 0: K (lower tiles of size T incl. full diagonal tiles, + noise on the
 //         global diagonal); mode 1: cross / prior (all entries, no noise).
 // out32 (optional): the same entries rounded to FP32 (mixed path).
-template <int MODE, typename OutT>
+// AR: rows per CTA.
+template <int MODE, typename OutT, int AR>
 __global__ void __launch_bounds__(AC) se_kernel(const double *__restrict__ xrow,
                                                int rows,
                                                const double *__restrict__ xcol,
@@ -260,10 +260,14 @@ __global__ void reduce_rows_kernel(const double *__restrict__ part, int m, int p
     }
 }
 
-size_t se_smem(int d, bool per_row)
+constexpr int AR_MANY = 64;
+constexpr int AR_FEW = 16;
+constexpr int64_t SE_MANY_CTAS = 4096;  // of 64 rows
+
+size_t se_smem(int d, bool per_row, int ar)
 {
-    const size_t xr = per_row ? static_cast<size_t>(AR) * d : static_cast<size_t>(AR + d);
-    return (xr + AC + d + 2 * AR * (AC / 32)) * sizeof(double);
+    const size_t xr = per_row ? static_cast<size_t>(ar) * d : static_cast<size_t>(ar + d);
+    return (xr + AC + d + 2 * ar * (AC / 32)) * sizeof(double);
 }
 
 template <int MODE, typename OutT>
@@ -275,18 +279,27 @@ void launch_se(const double *xrow, int rows, const double *xcol, int cols, int d
     {
         return;
     }
-    size_t smem = se_smem(d, row_offsets != nullptr);
-    if (smem > 227 * 1024)
+    if (se_smem(d, row_offsets != nullptr, AR_MANY) > 227 * 1024)
     {
         throw Error(1, "too many regressors for the assembly kernel");
     }
+    // Entries summed directly don't depend on the rows a CTA takes: 16, where 64
+    // leave the SMs few CTAs, each a serial walk of its rows.  K of n = 1024 / 2048
+    // / 3250 / 4096 / 5120 / 8192 at d = 8: 8.7 / 16.7 / 28.9 / 42.8 / 63.8 / - us
+    // with 16 rows, 19.5 / 26.2 / 47.2 / 56.8 / 67.9 / 153 with 64, whose windows
+    // serve more rows.
+    const bool recur = d >= RECUR_MIN_D && row_offsets == nullptr;
+    const bool few = !recur && static_cast<int64_t>(ceil_div(cols, AC)) * ceil_div(rows, AR_MANY) < SE_MANY_CTAS;
+    const int ar = few ? AR_FEW : AR_MANY;
+    const size_t smem = se_smem(d, row_offsets != nullptr, ar);
+    const auto kern = few ? se_kernel<MODE, OutT, AR_FEW> : se_kernel<MODE, OutT, AR_MANY>;
     if (smem > 48 * 1024)
     {
-        ensure_smem_attr(reinterpret_cast<const void *>(se_kernel<MODE, OutT>), static_cast<int>(smem));
+        ensure_smem_attr(reinterpret_cast<const void *>(kern), static_cast<int>(smem));
     }
-    dim3 grid(ceil_div(cols, AC), ceil_div(rows, AR));
-    se_kernel<MODE, OutT><<<grid, AC, smem, s>>>(xrow, rows, xcol, cols, d, T, p, out, ldo, alpha, mean_partial,
-                                                 parts, row_offsets, out32, ld32);
+    dim3 grid(ceil_div(cols, AC), ceil_div(rows, ar));
+    kern<<<grid, AC, smem, s>>>(xrow, rows, xcol, cols, d, T, p, out, ldo, alpha, mean_partial, parts, row_offsets,
+                                out32, ld32);
     GPRAT_LAUNCH_CHECK();
 }
 

@@ -29,3 +29,19 @@ def test_every_tiling_holds_the_same_factor():
         factors.append(np.tril(L))
     for L in factors[1:]:
         assert np.array_equal(L, factors[0])
+
+
+def test_entries_do_not_depend_on_the_rows_a_cta_takes():
+    """With one tile the strict upper triangle holds K itself: matrices that are
+    assembled 16 and 64 rows at a time agree where they share the series."""
+    from gprat_b200 import capi
+
+    rng = np.random.default_rng(6)
+    x, y = rng.standard_normal(6160), rng.standard_normal(6160)
+    upper = {}
+    for n in (6144, 5120, 1027, 15):
+        gp = capi.CudaGP(x[:n + 7], y[:n], 1, n, n_reg=8)
+        upper[n] = np.triu(gp.cholesky([1.0, 1.0, 0.1])[0].reshape(n, n), 1)
+        gp.close()
+    for n in (5120, 1027, 15):
+        assert np.array_equal(upper[n], upper[6144][:n, :n])
