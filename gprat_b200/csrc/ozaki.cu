@@ -6,8 +6,8 @@
 // rows at once into registers (so the block's DRAM latency is paid once, not
 // per row), finds the row maxima and, across the CTA, the block maximum,
 // and writes s digit planes from the registers, 4 bytes per lane and plane
-// (128-byte rows).  Digits
-// are peeled with the 1.5 * 2^52 rounding trick: y = t + 1.5 * 2^52 rounds t
+// (128-byte rows).  Up to five digits come straight from the value
+// (direct_digit); more are peeled with the 1.5 * 2^52 rounding trick: y = t + 1.5 * 2^52 rounds t
 // to the nearest integer d (ties to even), d is the low word of y, then
 // t <- (t - d) * 254 (t - d is exact; the product rounds only once the
 // remainder has used up the 53 bits), so D_0 .. D_{s-1} are the leading s
@@ -42,7 +42,8 @@
 //     block's exponents are loaded while a block is read.  After the tile's
 //     last unit, alpha * acc (+ C, whose lines were sent for when the tile
 //     began) is written 16 columns at a time through 4 KB of shared memory per
-//     warp, whole 128-byte lines at once.
+//     warp, whole 128-byte lines at once; on request the digits of the first
+//     128 columns are written from the registers instead or as well.
 // What bounds it: the epilogue.  FP64 instructions take 3.2 times as long
 // while int8 MMAs stream (12 cycles a warp instruction and scheduler instead
 // of 4), and so do integer ones between them, so what counts is the FP64
