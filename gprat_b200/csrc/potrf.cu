@@ -179,7 +179,7 @@ constexpr double MIN_PIVOT = 1e-290;
 // whose operands but the last are ready one step earlier.  FAST false (entries
 // out of the seeds' range): divisions.
 template <bool FAST>
-__device__ __forceinline__ void pivot_chain(double *a, int c0, bool wait_tile, double *u, double *piv, double *pinv)
+__device__ __forceinline__ void pivot_chain(double *a, int c0, double *u, double *piv, double *pinv)
 {
     const int lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
@@ -189,10 +189,6 @@ __device__ __forceinline__ void pivot_chain(double *a, int c0, bool wait_tile, d
         if (h == 1)
         {
             // the last 16 x 16 tile: A22 -= (U21 D^-1) U21^T
-            if (wait_tile)
-            {
-                bar_sync(HALF_BAR, 64);
-            }
             double *c = a + (c0 + HB + g) * PS + c0 + HB + 2 * t;
             double af[2][4], bf[2][2][2], cf[2][4];
 #pragma unroll
@@ -728,15 +724,21 @@ __global__ void __launch_bounds__(PTHREADS, 1) potrf_inv_kernel(T *A, int64_t ld
         double *u = ubuf + (s & 1) * SB * US;
         if (warp == 0)
         {
+            // the sub-block is complete once the product warp has updated its last
+            // 16 x 16 tile: neither the test below nor the chain may look at it before
+            if (s > 0)
+            {
+                bar_sync(HALF_BAR, 64);
+            }
             if (__all_sync(0xffffffffu, seeds_apply(sa[(c0 + lane) * PS + c0 + lane])))
             {
                 min_pivot = MIN_PIVOT;
-                pivot_chain<true>(sa, c0, s > 0, u, piv + c0, pinv + c0);
+                pivot_chain<true>(sa, c0, u, piv + c0, pinv + c0);
             }
             else
             {
                 min_pivot = 0.0;
-                pivot_chain<false>(sa, c0, s > 0, u, piv + c0, pinv + c0);
+                pivot_chain<false>(sa, c0, u, piv + c0, pinv + c0);
             }
         }
         else if (warp == CHASE_WARP)
