@@ -89,6 +89,7 @@ def _load() -> ctypes.CDLL:
                                                _dp, _dp, ctypes.c_int, _dp, _dp, ctypes.c_int]
     lib.gprat_cu_test_dgemm_solve.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_int, _dp, _dp, _dp, _dp, _dp,
                                               ctypes.c_int]
+    lib.gprat_cu_test_pivot_reciprocals.argtypes = [ctypes.c_int, _dp, _dp, _dp, _dp]
     lib.gprat_cu_test_set_wait_budget.argtypes = [_i64]
     _i8p, _i32p = ctypes.POINTER(ctypes.c_int8), ctypes.POINTER(ctypes.c_int32)
     lib.gprat_cu_test_oz_split.argtypes = [ctypes.c_int, ctypes.c_int, _dp, ctypes.c_int, ctypes.c_int, _i8p, _i32p]
@@ -222,6 +223,14 @@ def test_dgemm_solve(P0: np.ndarray, P1: np.ndarray, Linv: np.ndarray, rowsq: Op
     check(lib.gprat_cu_test_dgemm_solve(P0.shape[0], P1.shape[0], Linv.shape[0], _p(P0), _p(P1), _p(Linv),
                                         _p(rowsq) if rowsq is not None else None,
                                         _p(y) if y is not None else None, int(tile)))
+
+
+def test_pivot_reciprocals(d: np.ndarray) -> Tuple[np.ndarray, np.ndarray, np.ndarray]:
+    """The reciprocals of the diagonal block's pivots: (the approximation they start from, the result, 1 / d)."""
+    d = _arr(d)
+    seed, inv, quotient = np.empty_like(d), np.empty_like(d), np.empty_like(d)
+    check(lib.gprat_cu_test_pivot_reciprocals(d.size, _p(d), _p(seed), _p(inv), _p(quotient)))
+    return seed, inv, quotient
 
 
 def test_trsv(kind: int, L: np.ndarray, b: np.ndarray, max_ctas: int = 0) -> Tuple[np.ndarray, np.ndarray]:

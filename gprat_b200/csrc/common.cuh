@@ -244,6 +244,9 @@ void potrf_diag(double *A, int64_t lda, int bs, int row0, double *Linv, int64_t 
 // and the FP64 diagonal of L (diag, bs values).  Linv (FP64) may be null.
 void potrf_diag_f32(float *A, int64_t lda, int bs, int row0, double *Linv, int64_t ldi, float *Linv32, int64_t ldi32,
                     double *diag, DeviceStatus *status, cudaStream_t s, bool write_l = true);
+// The reciprocals of potrf_diag's chain, for n values: the approximation it starts
+// from, what it makes of it, and the quotient 1 / d.
+void pivot_reciprocals(const double *d, int n, double *seed, double *inv, double *quotient, cudaStream_t s);
 
 // Triangular solves with the blocked factor (L in Lmat, diagonal-block
 // inverses in Linv, block size nb).

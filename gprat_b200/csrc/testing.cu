@@ -626,3 +626,34 @@ extern "C" int gprat_cu_test_dgemm_solve(int m0, int m1, int bs, double *P0, dou
         return GPRAT_CU_ERR_INVALID_ARG;
     }
 }
+
+extern "C" int gprat_cu_test_pivot_reciprocals(int n, const double *d, double *seed, double *inv, double *quotient)
+{
+    try
+    {
+        if (n <= 0 || d == nullptr || seed == nullptr || inv == nullptr || quotient == nullptr)
+        {
+            throw Error(GPRAT_CU_ERR_INVALID_ARG, "gprat_cu_test_pivot_reciprocals: invalid arguments");
+        }
+        const size_t bytes = static_cast<size_t>(n) * 8;
+        Buf dd(bytes), ds(bytes), di(bytes), dq(bytes);
+        GPRAT_CUDA_CHECK(cudaMemcpy(dd.p, d, bytes, cudaMemcpyHostToDevice));
+        pivot_reciprocals(static_cast<double *>(dd.p), n, static_cast<double *>(ds.p), static_cast<double *>(di.p),
+                          static_cast<double *>(dq.p), nullptr);
+        GPRAT_CUDA_CHECK(cudaMemcpy(seed, ds.p, bytes, cudaMemcpyDeviceToHost));
+        GPRAT_CUDA_CHECK(cudaMemcpy(inv, di.p, bytes, cudaMemcpyDeviceToHost));
+        GPRAT_CUDA_CHECK(cudaMemcpy(quotient, dq.p, bytes, cudaMemcpyDeviceToHost));
+        set_last_error("");
+        return GPRAT_CU_OK;
+    }
+    catch (const Error &e)
+    {
+        set_last_error(e.what());
+        return e.code;
+    }
+    catch (const std::exception &e)
+    {
+        set_last_error(e.what());
+        return GPRAT_CU_ERR_INVALID_ARG;
+    }
+}

@@ -352,6 +352,13 @@ int gprat_cu_test_dgemm_solve(int m0,
                               int tile);
 
 /*
+ * Kernel-level test entry (no counterpart in the reference): the reciprocals of
+ * the diagonal block's pivots for n values d on the current device: the
+ * approximation they start from, the result, and CUDA's quotient 1 / d.
+ */
+int gprat_cu_test_pivot_reciprocals(int n, const double *d, double *seed, double *inv, double *quotient);
+
+/*
  * Kernel-level test entry (no counterpart in the reference): the
  * single-launch blocked triangular solves of the library on the current
  * device.  L: n x n row-major host matrix whose lower triangle (diagonal
