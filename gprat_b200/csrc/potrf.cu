@@ -150,12 +150,29 @@ __device__ __forceinline__ double rcp_series(double d, double y)
     return fma(e, e, e);
 }
 
-// The range the seeds (and the squares of a pivot column) are used in, by the
-// sub-block's current diagonal, which bounds its pivots and columns.  A pivot
-// that falls below MIN_PIVOT from there lost 170 decimal places to
-// cancellation and is reported like a non-positive one.
-__device__ __forceinline__ bool seeds_apply(double diag) { return diag > 1e-120 && diag < 1e150; }
-constexpr double MIN_PIVOT = 1e-290;
+// The chain wants pivots and their reciprocals to be normal numbers.  A block
+// whose largest diagonal entry, which bounds its pivots, is not within 2^+-RANGE is
+// therefore factored as 4^shift A, an exact multiple that brings that entry to [1,
+// 4): L = 2^-shift L', L^-1 = 2^shift L'^-1.  A pivot below 2^-1022 (1e-157 of
+// that entry or less) is reported like a non-positive one.  A block with an
+// infinity or a NaN on its diagonal, or nothing positive, has no such entry and
+// is eliminated with divisions.
+constexpr int RANGE = 500;
+constexpr double MIN_PIVOT = 2.2250738585072014e-308;  // 2^-1022
+
+// By the high word of the largest diagonal entry (0: nothing positive).
+__device__ __forceinline__ bool no_range(int top) { return top == 0 || top == 0x7ff00000; }
+__device__ __forceinline__ int range_shift(int top)
+{
+    const int e = (top >> 20) - 1023;
+    return no_range(top) || (e >= -RANGE && e < RANGE) ? 0 : -(e >> 1);
+}
+
+// v 2^e, |e| <= 512
+__device__ __forceinline__ double times_pow2(double v, int e)
+{
+    return e == 0 ? v : v * __hiloint2double((1023 + e) << 20, 0);
+}
 
 // Warp 0: A = L~ D L~^T of the 32 x 32 sub-block at (c0, c0), lane i holding row
 // i, 16 columns at a time; the last 16 x 16 tile is updated with the first 16
@@ -169,8 +186,8 @@ constexpr double MIN_PIVOT = 1e-290;
 // converged.
 // The chain from pivot to pivot, d' = a - u^2 / d on lane j+1 and a shuffle:
 // with 1 / d = y + y (e + e^2), d' = (a - u^2 y) - (u^2 y)(e + e^2), whose
-// operands but the last are ready one step earlier.  FAST false (entries
-// out of the seeds' range): divisions.
+// operands but the last are ready one step earlier (u^2 y as (u y) u: u^2 may
+// underflow where u^2 / d does not).  FAST false: divisions.
 template <bool FAST>
 __device__ __forceinline__ void pivot_chain(double *a, int c0, double *u, double *piv, double *pinv)
 {
@@ -243,8 +260,8 @@ __device__ __forceinline__ void pivot_chain(double *a, int c0, double *u, double
                 dinv = fma(y, ee, y);
                 if (jj + 1 < HB)
                 {
-                    const double q = r[jj] * r[jj] * y;
-                    dnext = fma(-q, ee, r[jj + 1] - q);
+                    const double w = r[jj] * y;
+                    dnext = fma(-(w * r[jj]), ee, fma(-w, r[jj], r[jj + 1]));
                 }
             }
             else if (jj + 1 < HB)
@@ -634,26 +651,54 @@ __global__ void __launch_bounds__(PTHREADS, 1) potrf_inv_kernel(T *A, int64_t ld
     double *pinv = piv + PB;             // [PB] their reciprocals
     double *rsq = pinv + PB;             // [PB] their reciprocal square roots (from the step after the pivots' on)
     __shared__ int bad;
-    __shared__ double min_pivot;
+    __shared__ int top_of[PB / 32];
     const int tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
     const bool mover = warp > CHASE_WARP && (warp & 3) == 0;
     const int mma_w = warp - 1 - (warp >> 2);                         // number among the product warps
     const int move_w = (warp >> 2) - 2, move_t = 32 * move_w + lane;  // among the data movers
-    const InverseOut out{ Linv, ldi, Linv32, ldi32, bs };
     if (tid == 0)
     {
         bad = 0;
     }
     pdl_wait();  // the previous kernel's results are visible from here on
     const bool al = aligned16(A, lda);
+    const double diag = tid < bs ? static_cast<double>(A[tid * (lda + 1)]) : 0.0;
     // the first sub-block's rows ahead of the rest: its chain starts on them
     load_rows<0, SB>(A, lda, al, bs, sa);
     asm volatile("cp.async.commit_group;\n" ::: "memory");
     load_rows<SB, PB>(A, lda, al, bs, sa);
     asm volatile("cp.async.commit_group;\ncp.async.wait_group 1;\n" ::: "memory");
+    if (warp < PB / 32)
+    {
+        // the high words of positive numbers are in the numbers' order
+        const int hi = __double2hiint(diag);
+        const int key = (hi & 0x7ff00000) == 0x7ff00000 ? 0x7ff00000 : diag > 0.0 ? max(hi, 1) : 0;
+        const int top = __reduce_max_sync(0xffffffffu, key);
+        if (lane == 0)
+        {
+            top_of[warp] = top;
+        }
+    }
     __syncthreads();
+    // (read again where it is needed: the chain leaves no registers to keep it in)
+    auto top = [&]() { return max(max(top_of[0], top_of[1]), max(top_of[2], top_of[3])); };
+    // (an FP32 block's numbers are in range)
+    if (const int shift = sizeof(T) == 8 ? range_shift(top()) : 0; shift != 0)
+    {
+        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        __syncthreads();
+        for (int i = warp; i < bs; i += NWARPS)
+        {
+            for (int c = lane; c <= i; c += 32)
+            {
+                sa[i * PS + c] = times_pow2(times_pow2(sa[i * PS + c], shift), shift);
+            }
+        }
+        __syncthreads();
+    }
+    const InverseOut out{ Linv, ldi, Linv32, ldi32, bs };
 
     // L's sub-block s (its columns u scaled by 1 / sqrt(d)) and diagonal, to
     // memory, by this thread as number me of count
@@ -683,7 +728,7 @@ __global__ void __launch_bounds__(PTHREADS, 1) potrf_inv_kernel(T *A, int64_t ld
     {
         const double d = piv[s * SB + lane];
         rsq[s * SB + lane] = rsqrt(d);
-        const unsigned wrong = __ballot_sync(0xffffffffu, !(d > min_pivot) && s * SB + lane < bs);
+        const unsigned wrong = __ballot_sync(0xffffffffu, !(no_range(top()) ? d > 0.0 : d >= MIN_PIVOT) && s * SB + lane < bs);
         if (lane == 0 && wrong != 0 && bad == 0)
         {
             bad = row0 + s * SB + __ffs(wrong);
@@ -716,20 +761,16 @@ __global__ void __launch_bounds__(PTHREADS, 1) potrf_inv_kernel(T *A, int64_t ld
         double *u = ubuf + (s & 1) * SB * US;
         if (warp == 0)
         {
-            // the sub-block is complete once the product warp has updated its last
-            // 16 x 16 tile: neither the test below nor the chain may look at it before
             if (s > 0)
             {
-                bar_sync(HALF_BAR, 64);
+                bar_sync(HALF_BAR, 64);  // the sub-block's last 16 x 16 tile is updated
             }
-            if (__all_sync(0xffffffffu, seeds_apply(sa[(c0 + lane) * PS + c0 + lane])))
+            if (!no_range(top()))
             {
-                min_pivot = MIN_PIVOT;
                 pivot_chain<true>(sa, c0, u, piv + c0, pinv + c0);
             }
             else
             {
-                min_pivot = 0.0;
                 pivot_chain<false>(sa, c0, u, piv + c0, pinv + c0);
             }
         }
@@ -911,6 +952,27 @@ __global__ void __launch_bounds__(PTHREADS, 1) potrf_inv_kernel(T *A, int64_t ld
     inverse_row_block(out, sa, false, xall + 3 * SB * XS, rsq, tbuf, 3, warp, NWARPS, g, t);
     write_xs(3, false, tid, PTHREADS);
     write_diag(3, tid, PTHREADS);
+    if (const int shift = sizeof(T) == 8 ? range_shift(top()) : 0; shift != 0)
+    {
+        // (rare) what has been written, L' and its inverse, to the block's own scale
+        __syncthreads();
+        for (int i = warp; i < bs; i += NWARPS)
+        {
+            for (int c = lane; c <= i; c += 32)
+            {
+                if (write_l)
+                {
+                    T &l = A[static_cast<int64_t>(i) * lda + c];
+                    l = static_cast<T>(times_pow2(static_cast<double>(l), -shift));
+                }
+                if (Linv != nullptr)
+                {
+                    double &x = Linv[static_cast<int64_t>(i) * ldi + c];
+                    x = times_pow2(x, shift);
+                }
+            }
+        }
+    }
 }
 
 __global__ void reciprocal_kernel(const double *__restrict__ d, int n, double *__restrict__ seed,
