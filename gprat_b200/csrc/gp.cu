@@ -436,6 +436,45 @@ void gradient_device(gprat_cu_gp *gp, bool adam, cudaStream_t s)
     adjoint_finish(gp->partials.ptr, np, gp->n, gp->params.ptr, adam, s);
 }
 
+// Factors the covariance and copies the tiles (i, 0) .. (i, i) of it to row(i).
+template <typename Row>
+void cholesky_rows(gprat_cu_gp *gp, const double hyper[3], const Row &row)
+{
+    DeviceGuard guard(gp->device);
+    StepPrefix prefix("cholesky_step");
+    upload_hyper(gp, hyper, gp->stream);
+    // The factor itself is the result, compared entry by entry with the
+    // reference's.  Subtracting the products one by one keeps the error of
+    // an entry that cancels to next to nothing in step with what is left of
+    // it: the smallest entries (1e-7 at n = 32768) agree with the
+    // reference's to 3e-11, against 5e-10 with sums subtracted, although
+    // those are closer over all entries (root mean square 7e-17 against
+    // 5e-16).
+    SolveRows none{};
+    none.c_first = true;
+    factor_fp64(gp, none, gp->stream);
+    finish_and_check(gp);
+    // The tiles are put in order on the device, a part of a tile row at a
+    // time, and copied straight to where they belong: copying the whole
+    // matrix into a host buffer of its own and from there tile by tile
+    // took twenty times as long as the factorisation at n = 2048.
+    constexpr int64_t PART = int64_t(1) << 23;  // 64 MB
+    const int T = gp->T, nt = gp->n_tiles;
+    const int part = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(PART / T, int64_t(nt) * T)));
+    gp->W.ensure(static_cast<int64_t>(part) * T);
+    for (int i = 0; i < nt; ++i)
+    {
+        const int64_t lines = static_cast<int64_t>(i + 1) * T;
+        for (int64_t l = 0; l < lines; l += part)
+        {
+            const int count = static_cast<int>(std::min<int64_t>(part, lines - l));
+            pack_lines(gp->K.ptr + static_cast<int64_t>(i) * T * gp->ld, gp->ld, T, l, count, gp->W.ptr, gp->stream);
+            download(gp, row(i) + l * T, gp->W.ptr, static_cast<int64_t>(count) * T);
+        }
+    }
+    GPRAT_CUDA_CHECK(cudaStreamSynchronize(gp->stream));
+}
+
 void check_gp(gprat_cu_gp *gp) { require(gp != nullptr, "GP handle is NULL"); }
 
 }  // namespace
@@ -890,42 +929,27 @@ int gprat_cu_cholesky(gprat_cu_gp *gp, const double hyper[3], double *tiles_out)
         {
             check_gp(gp);
             require(tiles_out != nullptr, "output must not be NULL");
-            DeviceGuard guard(gp->device);
-            StepPrefix prefix("cholesky_step");
-            upload_hyper(gp, hyper, gp->stream);
-            // The factor itself is the result, compared entry by entry with the
-            // reference's.  Subtracting the products one by one keeps the error of
-            // an entry that cancels to next to nothing in step with what is left of
-            // it: the smallest entries (1e-7 at n = 32768) agree with the
-            // reference's to 3e-11, against 5e-10 with sums subtracted, although
-            // those are closer over all entries (root mean square 7e-17 against
-            // 5e-16).
-            SolveRows none{};
-            none.c_first = true;
-            factor_fp64(gp, none, gp->stream);
-            finish_and_check(gp);
-            // The tiles are put in order on the device, a part of a tile row at a
-            // time, and copied straight to where they belong: copying the whole
-            // matrix into a host buffer of its own and from there tile by tile
-            // took twenty times as long as the factorisation at n = 2048.
-            constexpr int64_t PART = int64_t(1) << 23;  // 64 MB
-            const int T = gp->T, nt = gp->n_tiles;
-            const size_t tt = static_cast<size_t>(T) * T;
-            const int part = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(PART / T, int64_t(nt) * T)));
-            gp->W.ensure(static_cast<int64_t>(part) * T);
-            for (int i = 0; i < nt; ++i)
+            const size_t nt = gp->n_tiles, tt = static_cast<size_t>(gp->T) * gp->T;
+            cholesky_rows(gp, hyper, [&](size_t i) { return tiles_out + i * nt * tt; });
+            for (size_t i = 0; i < nt; ++i)
             {
-                double *row = tiles_out + static_cast<size_t>(i) * nt * tt;
-                const int64_t lines = static_cast<int64_t>(i + 1) * T;
-                for (int64_t l = 0; l < lines; l += part)
-                {
-                    const int count = static_cast<int>(std::min<int64_t>(part, lines - l));
-                    pack_lines(gp->K.ptr + static_cast<int64_t>(i) * T * gp->ld, gp->ld, T, l, count, gp->W.ptr, gp->stream);
-                    download(gp, row + l * T, gp->W.ptr, static_cast<int64_t>(count) * T);
-                }
-                std::memset(row + static_cast<size_t>(i + 1) * tt, 0, static_cast<size_t>(nt - i - 1) * tt * sizeof(double));
+                std::memset(tiles_out + (i * nt + i + 1) * tt, 0, (nt - i - 1) * tt * sizeof(double));
             }
-            GPRAT_CUDA_CHECK(cudaStreamSynchronize(gp->stream));
+        });
+}
+
+int gprat_cu_cholesky_rows(gprat_cu_gp *gp, const double hyper[3], double *const *rows_out)
+{
+    return guarded(
+        [&]
+        {
+            check_gp(gp);
+            require(rows_out != nullptr, "output must not be NULL");
+            for (int i = 0; i < gp->n_tiles; ++i)
+            {
+                require(rows_out[i] != nullptr, "a tile row's output must not be NULL");
+            }
+            cholesky_rows(gp, hyper, [&](size_t i) { return rows_out[i]; });
         });
 }
 

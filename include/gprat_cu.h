@@ -122,6 +122,11 @@ int gprat_cu_gp_set_int8_groups(gprat_cu_gp *gp, int factor_groups, int variance
  * (the reference returns them empty).
  */
 int gprat_cu_cholesky(gprat_cu_gp *gp, const double hyper[3], double *tiles_out);
+/*
+ * The lower tiles alone: the i + 1 tiles of tile row i, one after another, go to
+ * rows_out[i] (n_tiles pointers, to (i+1)*n_tile_size^2 doubles each).
+ */
+int gprat_cu_cholesky_rows(gprat_cu_gp *gp, const double hyper[3], double *const *rows_out);
 
 /* Predictive mean (gprat::GP::predict, core/src/gprat_c.cpp:106-154). */
 int gprat_cu_predict(gprat_cu_gp *gp,
