@@ -271,19 +271,16 @@ void trsv_fused_backward_f32(const float *L, int64_t ld, const float *Linv, int 
 // The same from b into x, whose bytes the caller has set to 0xFF and *ticket to
 // 0.  skip (optional, device): when *skip != 0 at launch the solve returns at
 // once (a preconditioner step of an already converged CG iteration).
-void trsv_forward_f32(const float *L, int64_t ld, const float *Linv, int n, const double *b, double *x, int *ticket,
-                      DeviceStatus *st, cudaStream_t s, int max_ctas, const int *skip);
-void trsv_backward_f32(const float *L, int64_t ld, const float *Linv, int n, const double *b, double *x, int *ticket,
-                       DeviceStatus *st, cudaStream_t s, int max_ctas, const int *skip);
+void trsv_prepared_forward_f32(const float *L, int64_t ld, const float *Linv, int n, const double *b, double *x,
+                               int *ticket, DeviceStatus *st, cudaStream_t s, int max_ctas, const int *skip);
+void trsv_prepared_backward_f32(const float *L, int64_t ld, const float *Linv, int n, const double *b, double *x,
+                                int *ticket, DeviceStatus *st, cudaStream_t s, int max_ctas, const int *skip);
 // Poll budget of the bounded waits on the current device: the single-launch
 // solves' on an unsolved block and the FP64 products' on their operand copies
 // (polls < 0: the defaults, about 0.5-1 s and 2 s).
 void set_wait_budget(long long polls);
 // The budget on the current device as the products take it (-1: the default).
 int wait_polls();
-// Same with an FP32 factor (mixed precision); FP64 right-hand side and arithmetic.
-void trsv_forward_f32(const float *L, int64_t ldl, const double *Linv, int nb, int n, double *rhs, cudaStream_t s);
-void trsv_backward_f32(const float *L, int64_t ldl, const double *Linv, int nb, int n, double *rhs, cudaStream_t s);
 
 // Loss 0.5*(y.a + sum log(L_ii^2) + n log 2pi)/n -> p->loss.
 void loss_kernel(const double *y, const double *alpha, const double *L, int64_t ldl, int n, DeviceParams *p,
@@ -295,7 +292,6 @@ void finalize_variance(const double *acc, int m, const DeviceParams *p, double *
 
 // Fill helpers
 void set_identity(double *A, int64_t lda, int n, cudaStream_t s);
-void copy_rows(const double *src, int64_t lds, double *dst, int64_t ldd, int rows, int cols, cudaStream_t s);
 
 // Adjoint (U: 16-byte aligned, even ldu): per lower tile partial sums of (Kinv - a a^T) .* dK for l and v, and
 // the noise term; then reduction + Adam (see optimizer.cu).

@@ -454,10 +454,10 @@ int blocks_for(int n) { return std::min(ceil_div(n, 256), 148 * 8); }
 // *skip != 0.
 void precondition(gprat_cu_gp *gp, const double *r, double *z, cudaStream_t s, int solve_ctas, const int *skip)
 {
-    trsv_forward_f32(gp->K32.ptr, gp->ld32, gp->Linv32.ptr, gp->n, r, gp->trsv_b.ptr, gp->flags.ptr, gp->status.ptr, s,
-                     solve_ctas, skip);
-    trsv_backward_f32(gp->K32.ptr, gp->ld32, gp->Linv32.ptr, gp->n, gp->trsv_b.ptr, z, gp->flags.ptr + 1,
-                      gp->status.ptr, s, solve_ctas, skip);
+    trsv_prepared_forward_f32(gp->K32.ptr, gp->ld32, gp->Linv32.ptr, gp->n, r, gp->trsv_b.ptr, gp->flags.ptr,
+                              gp->status.ptr, s, solve_ctas, skip);
+    trsv_prepared_backward_f32(gp->K32.ptr, gp->ld32, gp->Linv32.ptr, gp->n, gp->trsv_b.ptr, z, gp->flags.ptr + 1,
+                               gp->status.ptr, s, solve_ctas, skip);
 }
 
 }  // namespace

@@ -75,9 +75,7 @@ __global__ void __launch_bounds__(128) diag_bwd_kernel(const double *__restrict_
 
 // r[i] -= L[i][0:bs] . z for rows i in [0, rows) (L points at the block
 // column, rows start right below the diagonal block).  One warp per row.
-// L may be FP64 or FP32 (the mixed-precision factor); arithmetic is FP64.
-template <typename T>
-__global__ void __launch_bounds__(256) fwd_update_kernel(const T *__restrict__ L, int64_t ldl, int rows, int bs,
+__global__ void __launch_bounds__(256) fwd_update_kernel(const double *__restrict__ L, int64_t ldl, int rows, int bs,
                                                          const double *__restrict__ z, double *__restrict__ r)
 {
     __shared__ double zs[128];
@@ -92,11 +90,11 @@ __global__ void __launch_bounds__(256) fwd_update_kernel(const T *__restrict__ L
     {
         return;
     }
-    const T *lr = L + static_cast<int64_t>(row) * ldl;
+    const double *lr = L + static_cast<int64_t>(row) * ldl;
     double s = 0.0;
     for (int c = lane; c < bs; c += 32)
     {
-        s += static_cast<double>(lr[c]) * zs[c];
+        s += lr[c] * zs[c];
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
@@ -111,8 +109,7 @@ __global__ void __launch_bounds__(256) fwd_update_kernel(const T *__restrict__ L
 
 // r[c] -= sum_p L[p][c] * a[p] for c in [0, cols) (L points at the first
 // row of the block row; rows p < bs).  Threads own columns.
-template <typename T>
-__global__ void __launch_bounds__(256) bwd_update_kernel(const T *__restrict__ L, int64_t ldl, int cols, int bs,
+__global__ void __launch_bounds__(256) bwd_update_kernel(const double *__restrict__ L, int64_t ldl, int cols, int bs,
                                                          const double *__restrict__ a, double *__restrict__ r)
 {
     __shared__ double as[128];
@@ -129,7 +126,7 @@ __global__ void __launch_bounds__(256) bwd_update_kernel(const T *__restrict__ L
     double s = 0.0;
     for (int p = 0; p < bs; ++p)
     {
-        s += static_cast<double>(L[static_cast<int64_t>(p) * ldl + c]) * as[p];
+        s += L[static_cast<int64_t>(p) * ldl + c] * as[p];
     }
     r[c] -= s;
 }
@@ -195,11 +192,7 @@ __global__ void diag_ones_kernel(double *A, int64_t lda, int n)
 
 }  // namespace
 
-namespace
-{
-
-template <typename T>
-void trsv_forward_t(const T *L, int64_t ldl, const double *Linv, int nb, int n, double *rhs, cudaStream_t s)
+void trsv_forward(const double *L, int64_t ldl, const double *Linv, int nb, int n, double *rhs, double *, cudaStream_t s)
 {
     const int nblk = ceil_div(n, nb);
     for (int k = 0; k < nblk; ++k)
@@ -218,8 +211,8 @@ void trsv_forward_t(const T *L, int64_t ldl, const double *Linv, int nb, int n, 
     }
 }
 
-template <typename T>
-void trsv_backward_t(const T *L, int64_t ldl, const double *Linv, int nb, int n, double *rhs, cudaStream_t s)
+void trsv_backward(const double *L, int64_t ldl, const double *Linv, int nb, int n, double *rhs, double *,
+                   cudaStream_t s)
 {
     const int nblk = ceil_div(n, nb);
     for (int k = nblk - 1; k >= 0; --k)
@@ -235,29 +228,6 @@ void trsv_backward_t(const T *L, int64_t ldl, const double *Linv, int nb, int n,
             GPRAT_LAUNCH_CHECK();
         }
     }
-}
-
-}  // namespace
-
-void trsv_forward(const double *L, int64_t ldl, const double *Linv, int nb, int n, double *rhs, double *, cudaStream_t s)
-{
-    trsv_forward_t(L, ldl, Linv, nb, n, rhs, s);
-}
-
-void trsv_backward(const double *L, int64_t ldl, const double *Linv, int nb, int n, double *rhs, double *,
-                   cudaStream_t s)
-{
-    trsv_backward_t(L, ldl, Linv, nb, n, rhs, s);
-}
-
-void trsv_forward_f32(const float *L, int64_t ldl, const double *Linv, int nb, int n, double *rhs, cudaStream_t s)
-{
-    trsv_forward_t(L, ldl, Linv, nb, n, rhs, s);
-}
-
-void trsv_backward_f32(const float *L, int64_t ldl, const double *Linv, int nb, int n, double *rhs, cudaStream_t s)
-{
-    trsv_backward_t(L, ldl, Linv, nb, n, rhs, s);
 }
 
 void loss_kernel(const double *y, const double *alpha, const double *L, int64_t ldl, int n, DeviceParams *p,
@@ -289,12 +259,6 @@ void set_identity(double *A, int64_t lda, int n, cudaStream_t s)
     GPRAT_CUDA_CHECK(cudaMemset2DAsync(A, lda * sizeof(double), 0, n * sizeof(double), n, s));
     diag_ones_kernel<<<ceil_div(n, 256), 256, 0, s>>>(A, lda, n);
     GPRAT_LAUNCH_CHECK();
-}
-
-void copy_rows(const double *src, int64_t lds, double *dst, int64_t ldd, int rows, int cols, cudaStream_t s)
-{
-    GPRAT_CUDA_CHECK(cudaMemcpy2DAsync(dst, ldd * sizeof(double), src, lds * sizeof(double), cols * sizeof(double),
-                                       rows, cudaMemcpyDeviceToDevice, s));
 }
 
 }  // namespace gprat_cu

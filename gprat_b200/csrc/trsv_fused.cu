@@ -939,12 +939,12 @@ void trsv_fused_backward(const double *L, int64_t ld, const double *Linv, int n,
     bwd(L, ld, Linv, n, x, flags, scratch, st, s, max_ctas);
 }
 
-void trsv_forward_f32(const float *L, int64_t ld, const float *Linv, int n, const double *b, double *x, int *ticket,
-                      DeviceStatus *st, cudaStream_t s, int max_ctas, const int *skip)
+void trsv_prepared_forward_f32(const float *L, int64_t ld, const float *Linv, int n, const double *b, double *x,
+                               int *ticket, DeviceStatus *st, cudaStream_t s, int max_ctas, const int *skip)
 {
     if ((ld & 3) != 0 || (reinterpret_cast<uintptr_t>(L) & 15) != 0 || (reinterpret_cast<uintptr_t>(Linv) & 15) != 0)
     {
-        throw Error(1, "trsv_forward_f32: L and Linv must be 16-byte aligned, ld a multiple of 4");
+        throw Error(1, "trsv_prepared_forward_f32: L and Linv must be 16-byte aligned, ld a multiple of 4");
     }
     ensure_smem_attr(reinterpret_cast<const void *>(trsv_fwd_f32_kernel), static_cast<int>(SMEM_F32_FWD));
     trsv_fwd_f32_kernel<<<grid_for(ceil_div(n, FB), max_ctas), FT, SMEM_F32_FWD, s>>>(L, ld, Linv, n, b, x, ticket, st,
@@ -952,12 +952,12 @@ void trsv_forward_f32(const float *L, int64_t ld, const float *Linv, int n, cons
     GPRAT_LAUNCH_CHECK();
 }
 
-void trsv_backward_f32(const float *L, int64_t ld, const float *Linv, int n, const double *b, double *x, int *ticket,
-                       DeviceStatus *st, cudaStream_t s, int max_ctas, const int *skip)
+void trsv_prepared_backward_f32(const float *L, int64_t ld, const float *Linv, int n, const double *b, double *x,
+                                int *ticket, DeviceStatus *st, cudaStream_t s, int max_ctas, const int *skip)
 {
     if ((ld & 3) != 0 || (reinterpret_cast<uintptr_t>(L) & 15) != 0 || (reinterpret_cast<uintptr_t>(Linv) & 15) != 0)
     {
-        throw Error(1, "trsv_backward_f32: L and Linv must be 16-byte aligned, ld a multiple of 4");
+        throw Error(1, "trsv_prepared_backward_f32: L and Linv must be 16-byte aligned, ld a multiple of 4");
     }
     const int nblk = ceil_div(n, FB);
     ensure_smem_attr(reinterpret_cast<const void *>(trsv_bwd_f32_kernel), static_cast<int>(SMEM_F32_BWD));
@@ -969,25 +969,26 @@ void trsv_fused_forward_f32(const float *L, int64_t ld, const float *Linv, int n
                             double *scratch, DeviceStatus *st, cudaStream_t s, int max_ctas)
 {
     prepare(x, scratch, n, flags, s);
-    trsv_forward_f32(L, ld, Linv, n, scratch, x, flags, st, s, max_ctas, nullptr);
+    trsv_prepared_forward_f32(L, ld, Linv, n, scratch, x, flags, st, s, max_ctas, nullptr);
 }
 
 void trsv_fused_backward_f32(const float *L, int64_t ld, const float *Linv, int n, double *x, int *flags,
                              double *scratch, DeviceStatus *st, cudaStream_t s, int max_ctas)
 {
     prepare(x, scratch, n, flags, s);
-    trsv_backward_f32(L, ld, Linv, n, scratch, x, flags, st, s, max_ctas, nullptr);
+    trsv_prepared_backward_f32(L, ld, Linv, n, scratch, x, flags, st, s, max_ctas, nullptr);
 }
 
-// Sets the poll budget of the solves' waits on the current device; polls < 0
-// restores the default.  Test use: a budget of 0 makes a wait on an unsolved
-// block give up at once (the status word's timeout flag), with no hang.
 namespace
 {
 constexpr int MAX_DEVICES = 64;
 std::atomic<int> g_wait_polls[MAX_DEVICES];  // budget + 1; 0: the default
 }  // namespace
 
+// Sets the poll budget of the bounded waits on the current device: the solves'
+// (on the device) and the FP64 products' (passed with each launch); polls < 0
+// restores the defaults.  Test use: with a budget of 0 a wait for something that
+// is not there yet gives up at once (the status word's timeout flag), with no hang.
 void set_wait_budget(long long polls)
 {
     int dev = 0;
