@@ -162,7 +162,7 @@ struct RowGroup
     int M;  // 0: no such rows
 };
 
-// C -= A B^T (dgemm.cu) for up to two row groups that share B (N x K, ldb), in
+// C -= A B^T (dgemm.cu) for one or two row groups that share B (N x K, ldb), in
 // one launch.  lower: of group 0 only C[i][j] with j <= i is written (M >= N).
 // y (optional): y -= B z as well (N and K values).
 struct UpdateArgs

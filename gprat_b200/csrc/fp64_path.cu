@@ -38,8 +38,10 @@ namespace
 // Blocks of 128 columns per outer panel.  Narrow panels shorten the chain, wide
 // ones make the large updates deeper.  1 / 2 / 4 blocks: fit and predict 364 /
 // 371 / 385 us at n = 1024, 1.35 / 1.39 / 1.51 ms at n = 3250; loss and gradient
-// 18.2 / 17.9 / 18.2 ms at n = 8192; fit and predict 80.1 / 77.0 / 76.4 ms at
-// n = 16384, 627 / - / 591 ms at n = 32768 (589 with 8).
+// 18.2 / 17.9 / 18.2 ms at n = 8192; fit and predict with 2 / 4 24.5 / 24.6 ms at n
+// = 10240, 37.8 / 37.7 at 12288, 55.1 / 54.8 at 14336, 76.8 / 76.4 at 16384 (80.1
+// with 1), 218.0 / 215.8 at 24576, - / 591 at 32768 (627 with 1, 589 with 8); runs
+// differ by 0.1 %.
 int panel_blocks(int n) { return knob("GPRAT_CU_FP64_PANEL_BLOCKS", n <= 4096 ? 1 : n <= 12288 ? 2 : 4, 1, 64); }
 
 double *kat(const gprat_cu_gp *gp, int r, int c) { return gp->K.ptr + static_cast<int64_t>(r) * gp->ld + c; }

@@ -130,7 +130,7 @@ struct gprat_cu_gp
     gprat_cu::DevBuf<int32_t> oz_lr_e, oz_lb_e, oz_inv_e, oz_p_e, oz_w_e, oz_wp_e;
     gprat_cu::DevBuf<double> Kx;
 
-    // the int8-emulated fit + predict pipeline captured as one CUDA graph,
+    // the fit + predict pipeline of the handle's mode captured as one CUDA graph,
     // replayed while its key (buffers, sizes, modes, knobs) holds; graph_seen
     // is the key of the last eager run, captured when it repeats
     cudaGraphExec_t graph = nullptr;

@@ -50,11 +50,12 @@
 // instructions per element and block: 2 here (5 groups), 6 when each pair of
 // groups is converted by itself.  One 256 x 128 x 128 block of 5 groups takes
 // 8400 cycles, of which its MMAs are 3840 (64 each); with the epilogue's
-// arithmetic left out 5400, with the integer sums alone 7100.  At 8192^3, 5
-// groups, 1785 -> 2085 TOP/s against two issuing threads that waited for the
-// barriers themselves and three pairs per block; lower 28672^2 x 2048: 1603 ->
-// 1940; 8192 x 128 x 1920: 96.2 -> 82 us; 8192 x 128 x 128: 25.6 -> 19.5 us; 3
-// groups 1293 -> 1460.  4 groups: 1680 to 1780 from run to run (before 1720).
+// arithmetic left out 5400, with the integer sums alone 7100.  Against two issuing
+// threads that waited for the barriers themselves and three pairs per block, both
+// timed in turn on one box (launches one by one): 8192^3, 5 groups, 1808 -> 2111
+// TOP/s; 3 groups 1301 -> 1500; 4 groups 1736 -> 1805; lower 28672^2 x 2048 1602 ->
+// 1955; 8192 x 128 x 1920 97 -> 86 us; 8192 x 128 x 128 21 to 24 -> 19 to 24 us.
+// (Rates below are of versions on the way here, each pair from one run.)
 // Every mbarrier wait is bounded (tcgen05_ptx.cuh); a wait that gives up
 // raises the CTA's abort flag, the roles leave their loops, TMA copies in
 // flight get 200 us to land, the MMA issuer drains, TMEM is freed and the
@@ -377,7 +378,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) oz_split_kernel(const double *s
 // ---------------------------------------------------------------------------
 // GEMM
 
-// warpgroup 0: warp 0 TMA, warps 1 and 2 MMA (warp 3 idle); warpgroups 1 and 2
+// warpgroup 0: warp 0 TMA, warp 1 MMA, warp 2 scout (warp 3 idle); warpgroups 1 and 2
 // (warps 4..11): epilogue.  The kernel launches with 168 registers a thread;
 // warpgroup 0 gives registers up (setmaxnreg) so that each epilogue thread
 // holds 224: 128 * 56 + 256 * 224 = 384 * 168.
@@ -391,7 +392,7 @@ constexpr int OZ_A_BYTES = 128 * 128;  // 128 rows x 128 digit bytes
 constexpr int OZ_B_BYTES = 64 * 128;   // this CTA's half of the 128 B rows
 // Slots of one A and one B digit plane: >= s + 1, so that the next block's first
 // planes load early, and a power of two, so that a slot's index is a mask (9
-// slots: 2030 TOP/s at 8192^3, 5 groups; 8: 2110).
+// slots 4 % slower at 8192^3, 5 groups).
 constexpr int OZ_RING = 8;
 constexpr int OZ_NACC = 4;             // int32 accumulators of 128 TMEM columns
 constexpr int OZ_NPHASE = 4;           // barriers of the epilogue's phases, in turn
@@ -408,8 +409,8 @@ constexpr int OZ_GROUP_M = 8;  // row tiles per group of the non-lower tile orde
 
 // Whether the epilogue sums a block's groups in 64-bit integers: where that
 // saves FP64 instructions enough to pay for its two widening multiplications.
-// 3 groups: 1405 TOP/s at 8192^3 against 1300 in pairs; 5: 2030 against 1800;
-// 4: 1615 against 1700, so pairs; above 5 the sum has more than 52 bits.
+// At 8192^3 against pairs: 3 groups 8 % faster, 5 groups 13 %; 4 groups 5 %
+// slower, so pairs; above 5 the sum has more than 52 bits.
 __host__ __device__ constexpr bool oz_sums(int G)
 {
     return G == 3 || G == 5;
@@ -751,8 +752,8 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
         // slot is free long before the block's end, and the next block's
         // planes, loaded in the same order, find it.  Everything between two MMAs
         // is a gap (an issue returns about when the MMA before has completed),
-        // so a block's MMAs are unrolled over descriptors made before it (1986
-        // -> 2025 TOP/s at 8192^3, 5 groups).  Descriptors advance from
+        // so a block's MMAs are unrolled over descriptors made before it (2 %
+        // faster at 8192^3, 5 groups).  Descriptors advance from
         // the ring bases (a slot is OZ_A_BYTES / 16 or OZ_B_BYTES / 16 units of
         // the descriptor's address field).
         const uint64_t adesc0 = sw128_desc(smem_u32(aring));

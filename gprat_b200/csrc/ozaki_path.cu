@@ -46,8 +46,11 @@ namespace
 int oz_panel_blocks(int n) { return knob("GPRAT_CU_OZ_PANEL_BLOCKS", n <= 8192 ? 4 : n <= 20480 ? 8 : 16, 1, 64); }
 
 // The SMs that the trailing update holds while the side stream factors the
-// next panel, in percent: as many as leave the panel chain hidden.  80 / 86 /
-// 92 %: n = 16384 31.6 / 31.9 / 32.4 ms, 32768 204.8 / 202.4 / 202.8.
+// next panel, in percent: as many as leave the panel chain hidden.  ms with 80 /
+// 86 %: n = 16384 30.8 / 31.1, 18432 39.5 / 39.6, 20480 65.6 / 65.5, 22528 80.2 /
+// 80.4, 24576 97.2 / 97.7, 28672 141.6 / 141.0, 32768 197.3 / 194.7; from 20480 to
+// 28672 (m = 8192) the two lie within what runs differ by (92 %: 1.6 % slower at
+// 16384, as 86 at 32768).
 int oz_main_percent(int n) { return sm_percent("GPRAT_CU_OZ_MAIN_PERCENT", n <= 20480 ? 80 : 86); }
 
 // Digit-plane operands of one handle (TMA maps built per call: cheap host work).

@@ -287,7 +287,10 @@ int gprat_cu_stats_read(int64_t *launches, int64_t *gemm_launches, double *gemm_
  * ..., core/src/cpu/gp_functions.cpp:29-678) plus "... alpha refinement" for
  * the mixed-precision alpha and "... loss".  When enabled, every phase of
  * every call is bracketed by CUDA events on the stream that runs it (device
- * time; the look-ahead's side stream is included in "cholesky").
+ * time; the look-ahead's side stream is included in "cholesky").  The FP64 mode
+ * then runs its phases one after another, so that each can be timed: without
+ * timers the solves of alpha and of the variances are part of the factorisation's
+ * launches, and the whole call takes less than the phases' sum.
  * gprat_cu_steps_csv writes "label,calls,total_ms,mean_ms" rows (NUL
  * terminated, truncated to cap) and the size it needs into *needed.
  */

@@ -1,10 +1,12 @@
 """Bounded device waits: the single-launch triangular solves wait for earlier
-row blocks by re-reading x (a sentinel marks unsolved entries).  With the
-poll budget shrunk to 0 (gprat_cu_test_set_wait_budget), a wait on an
-unsolved block gives up at once: the kernel sets the status word's timeout
-flag and finishes, and the call returns GPRAT_CU_ERR_TIMEOUT.  With the
-default budget restored, the same handle solves correctly again.  Only global
-memory is polled, so nothing is left in flight when a wait gives up.
+row blocks by re-reading x (a sentinel marks unsolved entries), the FP64
+products for the TMA copies of their operands.  With the poll budget shrunk
+to 0 (gprat_cu_test_set_wait_budget), a wait for something that is not there
+yet gives up at once: the kernel sets the status word's timeout flag and
+finishes, and the call returns GPRAT_CU_ERR_TIMEOUT.  With the default budget
+restored, the same handle solves correctly again.  The solves only poll global
+memory; a product whose wait gave up issues no further copy and gives those in
+flight 200 us to land before it ends.
 """
 import numpy as np
 import pytest
