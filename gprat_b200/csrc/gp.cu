@@ -751,7 +751,7 @@ int64_t gp_copy_fitted(gprat_cu_gp *dst, gprat_cu_gp *src)
     bytes += copy_buf(dst, dst->flags, src, src->flags, true);
     bytes += copy_buf(dst, dst->params, src, src->params, true);
     bytes += copy_buf(dst, dst->status, src, src->status, true);
-    // per-batch predict working set: same capacity, no contents
+    // working set of a predict batch and of a fit: same capacity, no contents
     for (auto pr : { std::make_pair(&dst->xt, &src->xt), std::make_pair(&dst->W, &src->W),
                      std::make_pair(&dst->vacc, &src->vacc), std::make_pair(&dst->mean_part, &src->mean_part),
                      std::make_pair(&dst->mean, &src->mean), std::make_pair(&dst->var, &src->var) })
@@ -765,6 +765,7 @@ int64_t gp_copy_fitted(gprat_cu_gp *dst, gprat_cu_gp *src)
     copy_buf(dst, dst->oz_w_e, src, src->oz_w_e, false);
     copy_buf(dst, dst->oz_wp_e, src, src->oz_wp_e, false);
     copy_buf(dst, dst->Kx, src, src->Kx, false);
+    copy_buf(dst, dst->z, src, src->z, false);
     GPRAT_CUDA_CHECK(cudaStreamSynchronize(dst->stream));
     dst->pcg_last_iters = src->pcg_last_iters;
     return bytes;
